@@ -1,4 +1,6 @@
-// CUDA-core convolution passes of the diffusion step (sm_100a).
+// CUDA-core convolution passes of the diffusion step: those of the 16-bit fields and, for
+// some radii, the FP32 field's x pass (contig_pass; its other passes are in
+// stream_f32.cuh), and the generic pass.
 //
 // One repetition of the reference step (src/lib/cpp/cpu/diffusion.cc:314-320)
 // is three 1-D zero-boundary convolutions -- z, then y, then x -- followed by
@@ -26,6 +28,14 @@
 namespace maxi {
 
 template <int R> struct Taps { float k[2 * R + 1]; };
+
+// Programmatic dependent launch: the next pass's blocks may take free SM slots at once and
+// wait in pass_begin() until this pass is complete and its writes are visible.  Without the
+// launch attribute both instructions do nothing.
+__device__ __forceinline__ void pass_begin() {
+    asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+    asm volatile("griddepcontrol.wait;" ::: "memory");
+}
 
 // ---- strided (z / y) pass -------------------------------------------------
 constexpr int kStrTI = 32;    // inner columns per CTA (one warp wide)
@@ -162,7 +172,8 @@ template <int R> constexpr int contig_smem_bytes() { return kConTR * contig_stri
 // re-illuminated and rounded with error feedback along x in registers (the
 // carry restarts after every mask voxel, which is stored as exactly 1.0).
 template <int R, typename S, int MASK_FMT, bool FINAL, bool EF = false>
-__global__ void __launch_bounds__(kConThreads, (sizeof(S) == 4 && !FINAL && R <= 32) ? 5 : 1)
+// FP32, which runs at radii up to 32 only: five blocks per SM (48 registers).
+__global__ void __launch_bounds__(kConThreads, (sizeof(S) == 4 && !FINAL) ? 5 : 1)
 contig_pass(const S *__restrict__ in, S *__restrict__ out, const void *__restrict__ mask,
             uint16_t *__restrict__ out_u16, float *__restrict__ field_out,
             int64_t rows, int64_t nx, int64_t n_x_tiles, const Taps<R> taps) {
@@ -177,6 +188,7 @@ contig_pass(const S *__restrict__ in, S *__restrict__ out, const void *__restric
     const int tid = threadIdx.x;
     const int lane = tid & 31, warp = tid >> 5;
     constexpr int VEC = Vec16<S>::N;
+    pass_begin();
     // Vector path: full row block, rows and halo start on 16-byte boundaries, and
     // every output pointer aligned for 4-voxel vector access.  Chunks outside
     // [0, nx) are zero-filled (chunks never straddle the row ends).

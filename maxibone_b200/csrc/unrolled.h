@@ -46,6 +46,10 @@ template <typename S>
 cudaError_t dispatch_unrolled(const Volume &v, const void *mask, int mask_fmt, const float *kernel, int radius,
                               int64_t reps, S *b0, S *b1, uint16_t *out_u16, float *field_out, int32_t flags,
                               cudaStream_t st, const RunOpts &o = RunOpts{});
+template <>  // streaming passes (passes_f32.cu)
+cudaError_t dispatch_unrolled<float>(const Volume &v, const void *mask, int mask_fmt, const float *kernel, int radius,
+                                     int64_t reps, float *b0, float *b1, uint16_t *out_u16, float *field_out,
+                                     int32_t flags, cudaStream_t st, const RunOpts &o);
 
 // maxi_diffusion_device() with the RunOpts of an out-of-core slab.
 int diffusion_device_shrinking(const void *mask, int32_t mask_format, int64_t nz, int64_t ny, int64_t nx,

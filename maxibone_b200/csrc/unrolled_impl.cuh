@@ -1,5 +1,6 @@
-// Unrolled CUDA-core repetition loop (template definitions); included by the
-// per-type instantiation units passes_f32.cu, passes_bf16.cu, passes_f16.cu.
+// Repetition loop of the 16-bit fields: tensor-core passes, or the unrolled CUDA-core
+// passes (template definitions); included by the per-type units passes_bf16.cu and
+// passes_f16.cu (the FP32 field's loop is in passes_f32.cu).
 #pragma once
 
 #include "passes.cuh"
@@ -38,7 +39,7 @@ static cudaError_t set_smem(F *f, int bytes) {
 
 // One repetition loop for bucket radius R.  EF: error-feedback rounding of the
 // 16-bit storage type (see passes.cuh); use_tc: z and y passes on the tensor
-// cores (16-bit storage only, tc_pass.cu).
+// cores (tc_pass.cu).
 template <int R, typename S, bool EF>
 static cudaError_t run_unrolled(const Volume &v, const void *mask, int mask_fmt, const float *kernel,
                                 int radius, int64_t reps, S *buf0, S *buf1, uint16_t *out_u16,
@@ -108,47 +109,35 @@ static cudaError_t run_unrolled(const Volume &v, const void *mask, int mask_fmt,
         }
         {
             ProfScope ps(MAXI_KERNEL_Z, st);
-            if constexpr (sizeof(S) == 2) {
-                // After the first repetition the tensor-core x pass leaves the field in
-                // [y][z][x] row order (over all v.nz planes), which the z pass reads faster.
-                const tc::YzRows yz{buf0, v.nz, lo};
-                if (use_tc) e = tc::tc_strided<S>(b0, b1, nzv, v.ny, v.nx, true, kernel, radius, EF, st,
-                                                  tc_x && rep > 0 ? &yz : nullptr, hi_only);
-                else zy<<<zat * zit, kStrThreads, str_smem, st>>>(b0, b1, zA, zI, zat, zit, taps);
-            } else {
-                zy<<<zat * zit, kStrThreads, str_smem, st>>>(b0, b1, zA, zI, zat, zit, taps);
-            }
+            // After the first repetition the tensor-core x pass leaves the field in
+            // [y][z][x] row order (over all v.nz planes), which the z pass reads faster.
+            const tc::YzRows yz{buf0, v.nz, lo};
+            if (use_tc) e = tc::tc_strided<S>(b0, b1, nzv, v.ny, v.nx, true, kernel, radius, EF, st,
+                                              tc_x && rep > 0 ? &yz : nullptr, hi_only);
+            else zy<<<zat * zit, kStrThreads, str_smem, st>>>(b0, b1, zA, zI, zat, zit, taps);
         }
         if (e != cudaSuccess) return e;
         const bool last = rep + 1 == reps;
-        if constexpr (sizeof(S) == 2) {
-            if (yx) {
-                ProfScope ps(MAXI_KERNEL_YX, st);
-                const tc::YzRows yz{buf0, v.nz, lo};
-                e = tc::tc_yx<S>(b1, b0, mv, mask_fmt, last, last ? ou : nullptr, last ? fo : nullptr, nzv, v.ny,
-                                 v.nx, kernel, radius, EF, hi_only, st, &yz);
-                if (e != cudaSuccess) return e;
-                continue;
-            }
+        if (yx) {
+            ProfScope ps(MAXI_KERNEL_YX, st);
+            const tc::YzRows yz{buf0, v.nz, lo};
+            e = tc::tc_yx<S>(b1, b0, mv, mask_fmt, last, last ? ou : nullptr, last ? fo : nullptr, nzv, v.ny, v.nx,
+                             kernel, radius, EF, hi_only, st, &yz);
+            if (e != cudaSuccess) return e;
+            continue;
         }
         {
             ProfScope ps(MAXI_KERNEL_Y, st);
-            if constexpr (sizeof(S) == 2) {
-                if (use_tc) e = tc::tc_strided<S>(b1, b0, nzv, v.ny, v.nx, false, kernel, radius, EF, st, nullptr, hi_only);
-                else zy<<<yat * yit * yO, kStrThreads, str_smem, st>>>(b1, b0, yA, yI, yat, yit, taps);
-            } else {
-                zy<<<yat * yit * yO, kStrThreads, str_smem, st>>>(b1, b0, yA, yI, yat, yit, taps);
-            }
+            if (use_tc) e = tc::tc_strided<S>(b1, b0, nzv, v.ny, v.nx, false, kernel, radius, EF, st, nullptr, hi_only);
+            else zy<<<yat * yit * yO, kStrThreads, str_smem, st>>>(b1, b0, yA, yI, yat, yit, taps);
         }
         if (e != cudaSuccess) return e;
         {
             ProfScope ps(last ? MAXI_KERNEL_X_FINAL : MAXI_KERNEL_X, st);
             if (tc_x) {
-                if constexpr (sizeof(S) == 2) {
-                    const tc::YzRows yz{buf1, v.nz, lo};
-                    e = tc::tc_contig<S>(b0, b1, mv, mask_fmt, last, last ? ou : nullptr, last ? fo : nullptr, nzv,
-                                         v.ny, v.nx, kernel, radius, EF, st, &yz, hi_only);
-                }
+                const tc::YzRows yz{buf1, v.nz, lo};
+                e = tc::tc_contig<S>(b0, b1, mv, mask_fmt, last, last ? ou : nullptr, last ? fo : nullptr, nzv, v.ny,
+                                     v.nx, kernel, radius, EF, st, &yz, hi_only);
             } else if (!last) {
                 xpass<<<xt * xrb, kConThreads, con_smem, st>>>(b0, b1, mv, nullptr, nullptr, rows, v.nx, xt, taps);
             } else {
@@ -194,20 +183,16 @@ cudaError_t dispatch_unrolled(const Volume &v, const void *mask, int mask_fmt, c
     uint32_t *rebuild = (flags & MAXI_FLAG_MASK_FROM_FIELD) && mask_fmt == MAXI_MASK_BITPACKED
                             ? const_cast<uint32_t *>(static_cast<const uint32_t *>(mask))
                             : nullptr;
-    if constexpr (sizeof(S) == 2) {
-        // Error feedback relies on the following x pass to remove high-pass noise;
-        // kernels narrower than radius 4 (sigma < 1) pass too much of it.
-        const bool ef = (flags & MAXI_FLAG_NEAREST_ROUNDING) == 0 && radius >= 4;
-        const bool use_tc = (flags & MAXI_FLAG_NO_TENSOR_CORES) == 0 && tc::tc_supported(radius, v.nz, v.ny, v.nx);
-        // The rebuilt-mask semantics rewrite the mask between repetitions from the
-        // x pass's output; they keep the separate passes.
-        const bool fuse = (flags & (MAXI_FLAG_SEPARATE_PASSES | MAXI_FLAG_MASK_FROM_FIELD)) == 0;
-        const bool hi_only = tc::tc_single_set(radius, (flags & MAXI_FLAG_SPLIT_COEFFICIENTS) != 0);
-        if (ef) return dispatch_radius<S, true>(v, mask, mask_fmt, kernel, radius, reps, b0, b1, out_u16, field_out, use_tc, fuse, hi_only, rebuild, o, st);
-        return dispatch_radius<S, false>(v, mask, mask_fmt, kernel, radius, reps, b0, b1, out_u16, field_out, use_tc, fuse, hi_only, rebuild, o, st);
-    } else {
-        return dispatch_radius<S, false>(v, mask, mask_fmt, kernel, radius, reps, b0, b1, out_u16, field_out, false, false, false, rebuild, o, st);
-    }
+    // Error feedback relies on the following x pass to remove high-pass noise;
+    // kernels narrower than radius 4 (sigma < 1) pass too much of it.
+    const bool ef = (flags & MAXI_FLAG_NEAREST_ROUNDING) == 0 && radius >= 4;
+    const bool use_tc = (flags & MAXI_FLAG_NO_TENSOR_CORES) == 0 && tc::tc_supported(radius, v.nz, v.ny, v.nx);
+    // The rebuilt-mask semantics rewrite the mask between repetitions from the
+    // x pass's output; they keep the separate passes.
+    const bool fuse = (flags & (MAXI_FLAG_SEPARATE_PASSES | MAXI_FLAG_MASK_FROM_FIELD)) == 0;
+    const bool hi_only = tc::tc_single_set(radius, (flags & MAXI_FLAG_SPLIT_COEFFICIENTS) != 0);
+    if (ef) return dispatch_radius<S, true>(v, mask, mask_fmt, kernel, radius, reps, b0, b1, out_u16, field_out, use_tc, fuse, hi_only, rebuild, o, st);
+    return dispatch_radius<S, false>(v, mask, mask_fmt, kernel, radius, reps, b0, b1, out_u16, field_out, use_tc, fuse, hi_only, rebuild, o, st);
 }
 
 }  // namespace maxi
