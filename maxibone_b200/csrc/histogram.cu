@@ -14,21 +14,27 @@
 // counted voxel of a z-block adds to x_bins[x], y_bins[y], z_bins[z] and
 // r_bins[floor(sqrt((x-cx)^2 + (y-cy)^2))] at its voxel bin.
 //
-// Exact binning without FP64 in the kernels.  Each bin expression is a monotone
-// function of an integer value, so the host evaluates it with the reference's own
-// FP64 arithmetic for all 65536 values and keeps, per bin b, the threshold T[b] =
-// the smallest counted value whose bin is >= b.  A kernel estimates the bin in FP32
-// from the value's offset in the counted range and settles it with one comparison
-// each way against T (T[b] <= v < T[b+1] holds for exactly one b).  The host checks,
-// before any launch, that the estimate is within one bin for every counted value, so
-// the result is the reference's bin.  The tables are (bins + 1) words, L1-resident.
+// Exact binning without FP64 in the kernels.  Each bin expression is a monotone, very
+// nearly linear function of an integer value, so the host evaluates it with the reference's
+// own FP64 arithmetic for all 65536 values and fits a fixed-point line whose floor is the
+// reference's bin for every counted one (checked value by value): two integer instructions per
+// bin and no table.  Where no line fits, thresholds T[b] (the smallest counted value whose
+// bin is >= b) settle the fixed-point bin by one comparison each way.
 //
-// Counting.  One thread takes 8 consecutive voxels of a row (one 16-byte load when
-// rows are 16-byte aligned) and adds runs of equal keys once.  field_histogram
-// issues one 64-bit reduction per run into the histogram (L2-resident at the
-// pipeline's 2048 x 4096); each of its blocks walks one contiguous range of rows.  axis_histograms counts each row's voxel bins in a
-// shared-memory histogram with a list of the bins it touched, then adds those to
-// y_bins[y] and z_bins[z]; x and radial bins take one reduction per voxel.
+// Counting, field_histogram.  One thread takes 8 consecutive voxels of a row (one 16-byte load
+// when rows are 16-byte aligned), adds runs of equal keys once and issues one 64-bit
+// reduction per run into the histogram (L2-resident at the pipeline's 2048 x 4096); each
+// block walks one contiguous range of rows.
+//
+// Counting, axis_histograms.  L2 takes about 150 to 190 G reductions per second on random
+// cells, shared memory 2300 G (measured), and a voxel counts in four histograms.  So each
+// histogram has a kernel of its own whose blocks own a part of it in shared memory and read
+// the voxels that belong there: a y (or z) the rows of that y (or z), a strip of 8 x its
+// columns, a ring of radii its pixels.  Voxels are read four times and reductions go out once
+// per block and counted cell.  A 128 x 1024 x 1024 block at 4096 bins on a B200: z and y 98 us
+// each, x 155 (half of each 32-byte sector is another strip's), r 251 (a ring's row interval
+// fills about 40% of its sectors); before, one kernel with two reductions per voxel and a
+// shared histogram per row, 1611 us.
 #include <cmath>
 #include <mutex>
 #include <vector>
@@ -41,22 +47,25 @@ namespace {
 
 constexpr int kVec = 8;  // voxels per thread (one 16-byte load)
 
-// A counted value range [lo, lo + span] and its bin thresholds.
+// A counted value range [lo, lo + span] and the bin of each value in it.
 struct BinMap {
-    const uint32_t *T;  // T[0 .. bins]
+    const uint32_t *T;  // thresholds T[0 .. bins], or NULL where the fixed-point bin is exact
     int lo, span, bins;
-    float a, c;  // estimate: (v - lo) * a + c
+    uint32_t mul_lo, mul_hi;  // the bin's slope and offset in 1/2^32
+    uint64_t offset;
 };
 
-// The bin of v, or -1 if v is not counted.
+// The bin of v, or -1 if v is not counted.  EXACT: the map has no thresholds.
+template <bool EXACT = false>
 __device__ __forceinline__ int bin_of(const BinMap &m, int v) {
-    const unsigned d = (unsigned) (v - m.lo);
-    if (d > (unsigned) m.span) return -1;
-    int b = __float2int_rz(__fmaf_rn((float) d, m.a, m.c));
-    b = min(max(b, 0), m.bins - 1);
-    if ((uint32_t) v < __ldg(m.T + b)) b--;
-    else if ((uint32_t) v >= __ldg(m.T + b + 1)) b++;
-    return b;
+    const uint32_t d = (uint32_t) (v - m.lo);
+    int b = (int) (((uint64_t) d * m.mul_lo + m.offset) >> 32) + (int) (d * m.mul_hi);
+    if (!EXACT && m.T && d <= (uint32_t) m.span) {
+        b = min(max(b, 0), m.bins - 1);
+        if ((uint32_t) v < __ldg(m.T + b)) b--;
+        else if ((uint32_t) v >= __ldg(m.T + b + 1)) b++;
+    }
+    return d <= (uint32_t) m.span ? b : -1;
 }
 
 // Voxels are read once: loaded evict-first, so the L2-resident bins stay in L2.
@@ -127,25 +136,16 @@ __device__ __forceinline__ int64_t isqrt64(int64_t n) {
     return r;
 }
 
-// PRIV: the block keeps a shared histogram of the current row's voxel bins
-// (voxel_bins counters + voxel_bins touched-bin slots + a count) and adds it to
-// y_bins[y] and z_bins[z] at the end of the row; otherwise every voxel adds directly.
-// The row loop is block-uniform (it holds barriers).
-template <bool VEC8, bool PRIV>
-__global__ void axis_histograms_kernel(const uint16_t *__restrict__ voxels, int64_t nzl, int64_t Ny, int Nx,
+// axis_histograms where the shared-memory forms below do not apply: every voxel adds to the
+// global bins, runs of equal keys once (x: every voxel).
+template <bool VEC8>
+__global__ void axis_histograms_direct(const uint16_t *__restrict__ voxels, int64_t nzl, int64_t Ny, int Nx,
                                        int64_t z_start, int64_t y_start, int x_start, BinMap vm, int64_t cy,
                                        int64_t cx, unsigned long long *__restrict__ x_bins,
                                        unsigned long long *__restrict__ y_bins,
                                        unsigned long long *__restrict__ z_bins,
                                        unsigned long long *__restrict__ r_bins, int voxel_bins, int64_t n_r) {
     constexpr int V = VEC8 ? kVec : 1;
-    extern __shared__ uint32_t sh[];
-    uint32_t *hist = sh, *touched = sh + voxel_bins, *n_touched = sh + 2 * voxel_bins;
-    if (PRIV) {
-        for (int i = threadIdx.x; i < voxel_bins; i += blockDim.x) hist[i] = 0;
-        if (threadIdx.x == 0) *n_touched = 0;
-        __syncthreads();
-    }
     const int x_first = x_start / V * V;
     for (int64_t row = blockIdx.x; row < nzl * Ny; row += gridDim.x) {
         const int64_t zl = row / Ny, y = row - zl * Ny;
@@ -170,9 +170,6 @@ __global__ void axis_histograms_kernel(const uint16_t *__restrict__ voxels, int6
                     atomicAdd(x_bins + (int64_t) x * voxel_bins + vb, 1ull);
                     const int64_t r = isqrt64(dy2 + (x - cx) * (x - cx));
                     if (r < n_r) rk = r * voxel_bins + vb;
-                    if (PRIV) {
-                        if (atomicAdd(hist + vb, 1u) == 0) touched[atomicAdd(n_touched, 1u)] = (uint32_t) vb;
-                    }
                 }
                 if (rk == r_key) {
                     r_run++;
@@ -181,40 +178,186 @@ __global__ void axis_histograms_kernel(const uint16_t *__restrict__ voxels, int6
                     r_key = rk;
                     r_run = 1;
                 }
-                if (!PRIV) {
-                    if (vb == b_key) {
-                        b_run++;
-                    } else {
-                        if (b_key >= 0) {
-                            atomicAdd(yrow + b_key, (unsigned long long) b_run);
-                            atomicAdd(zrow + b_key, (unsigned long long) b_run);
-                        }
-                        b_key = vb;
-                        b_run = 1;
+                if (vb == b_key) {
+                    b_run++;
+                } else {
+                    if (b_key >= 0) {
+                        atomicAdd(yrow + b_key, (unsigned long long) b_run);
+                        atomicAdd(zrow + b_key, (unsigned long long) b_run);
                     }
+                    b_key = vb;
+                    b_run = 1;
                 }
             }
             if (r_key >= 0) atomicAdd(r_bins + r_key, (unsigned long long) r_run);
-            if (!PRIV && b_key >= 0) {
+            if (b_key >= 0) {
                 atomicAdd(yrow + b_key, (unsigned long long) b_run);
                 atomicAdd(zrow + b_key, (unsigned long long) b_run);
             }
         }
-        if (PRIV) {
-            __syncthreads();
-            const uint32_t n = *n_touched;
-            for (uint32_t i = threadIdx.x; i < n; i += blockDim.x) {
-                const uint32_t b = touched[i];
-                const unsigned long long c = hist[b];
-                hist[b] = 0;
-                atomicAdd(yrow + b, c);
-                atomicAdd(zrow + b, c);
+    }
+}
+
+// The block's counters, zeroed before and added to `bins` (the counted cells alone) after.
+__device__ __forceinline__ void counters_clear(uint32_t *c, int n) {
+    for (int i = threadIdx.x; i < n; i += blockDim.x) c[i] = 0;
+    __syncthreads();
+}
+__device__ __forceinline__ void counters_flush(const uint32_t *c, int n, unsigned long long *bins) {
+    __syncthreads();
+    for (int i = threadIdx.x; i < n; i += blockDim.x)
+        if (const uint32_t k = c[i]) atomicAdd(bins + i, (unsigned long long) k);
+}
+
+// y_bins or z_bins: block (p, chunk) counts the rows row0(p), row0(p) + row_step, .. of one y
+// (or z), from row chunk * per on, in one shared histogram.  A warp per row.
+struct RowSets {
+    int64_t sets, set_step, row_step, rows, first_row, per;  // per: rows of a chunk
+    int64_t first_set;                                      // sets below are not counted
+    unsigned long long *bins;                               // of set 0
+};
+template <bool VEC8, bool EXACT>
+__global__ void __launch_bounds__(256) row_set_histograms(const uint16_t *__restrict__ voxels, int Nx, int x_start,
+                                                          BinMap vm, RowSets s, int voxel_bins) {
+    extern __shared__ uint32_t counters[];
+    const int64_t set = s.first_set + blockIdx.x % (s.sets - s.first_set), chunk = blockIdx.x / (s.sets - s.first_set);
+    const int64_t end = min(s.rows, s.first_row + (chunk + 1) * s.per);
+    const int lane = threadIdx.x & 31;
+    counters_clear(counters, voxel_bins);
+    auto count = [&](int v) {
+        const int b = bin_of<EXACT>(vm, v);
+        if (b >= 0) atomicAdd(counters + b, 1u);
+    };
+    for (int64_t i = s.first_row + chunk * s.per + (threadIdx.x >> 5); i < end; i += blockDim.x >> 5) {
+        const uint16_t *row = voxels + (set * s.set_step + i * s.row_step) * Nx;
+        if (VEC8) {
+            // Up to x_first one voxel per lane, then two loads of 8 ahead of their counting.
+            const int x_first = (x_start + kVec - 1) / kVec * kVec;
+            if (x_start + lane < x_first) count(__ldcs(row + x_start + lane));
+            for (int x = x_first + lane * kVec; x < Nx; x += 64 * kVec) {
+                int v[kVec], w[kVec];
+                const bool second = x + 32 * kVec < Nx;
+                load_row8(row + x, v);
+                if (second) load_row8(row + x + 32 * kVec, w);
+#pragma unroll
+                for (int j = 0; j < kVec; j++) count(v[j]);
+                if (second)
+#pragma unroll
+                    for (int j = 0; j < kVec; j++) count(w[j]);
             }
-            __syncthreads();
-            if (threadIdx.x == 0) *n_touched = 0;
-            __syncthreads();
+        } else {
+            for (int x = x_start + lane; x < Nx; x += 32 * kVec) {
+                int v[kVec];
+#pragma unroll
+                for (int j = 0; j < kVec; j++) v[j] = x + 32 * j < Nx ? __ldcs(row + x + 32 * j) : -1;
+#pragma unroll
+                for (int j = 0; j < kVec; j++)
+                    if (v[j] >= 0) count(v[j]);
+            }
         }
     }
+    counters_flush(counters, voxel_bins, s.bins + set * voxel_bins);
+}
+
+// x_bins: block (strip, chunk) counts `strip` neighbouring x over the rows of the chunk, a
+// row per thread, two rows loaded ahead of their counting.
+template <bool VEC8, bool EXACT>
+__global__ void __launch_bounds__(1024) strip_histograms(const uint16_t *__restrict__ voxels, int64_t rows, int64_t Ny,
+                                                         int Nx, int64_t y_start, int x_start, BinMap vm, int strips,
+                                                         int strip, int64_t per, unsigned long long *__restrict__ x_bins,
+                                                         int voxel_bins) {
+    extern __shared__ uint32_t counters[];
+    const int x0 = blockIdx.x % strips * strip, width = min(strip, Nx - x0), skip = max(0, x_start - x0);
+    const int64_t begin = blockIdx.x / strips * per, end = min(rows, begin + per);
+    counters_clear(counters, width * voxel_bins);
+    auto count = [&](int v, int j) {
+        const int b = bin_of<EXACT>(vm, v);
+        if (b >= 0 && j >= skip) atomicAdd(counters + j * voxel_bins + b, 1u);
+    };
+    for (int64_t row = begin + threadIdx.x; row < end; row += 2 * blockDim.x) {
+        const int64_t next = row + blockDim.x;
+        bool first = true, second = next < end;
+        if (y_start > 0) {
+            first = row % Ny >= y_start;
+            second = second && next % Ny >= y_start;
+        }
+        const uint16_t *p = voxels + row * Nx + x0, *q = voxels + next * Nx + x0;
+        int v[kVec], w[kVec];
+        if (VEC8) {  // strips of 8
+            if (first) load_row8(p, v);
+            if (second) load_row8(q, w);
+        } else {
+#pragma unroll
+            for (int j = 0; j < kVec; j++) {
+                v[j] = first && j < width ? __ldg(p + j) : -1;
+                w[j] = second && j < width ? __ldg(q + j) : -1;
+            }
+        }
+        if (first)
+#pragma unroll
+            for (int j = 0; j < kVec; j++)
+                if (VEC8 || v[j] >= 0) count(v[j], j);
+        if (second)
+#pragma unroll
+            for (int j = 0; j < kVec; j++)
+                if (VEC8 || w[j] >= 0) count(w[j], j);
+    }
+    counters_flush(counters, width * voxel_bins, x_bins + (int64_t) x0 * voxel_bins);
+}
+
+// floor(sqrt(n)), 0 <= n < 2^31: the float estimate is within one.
+__device__ __forceinline__ int isqrt32(int n) {
+    int r = (int) sqrtf((float) n);
+    if ((uint32_t) r * (uint32_t) r > (uint32_t) n) r--;
+    if ((uint32_t) (r + 1) * (uint32_t) (r + 1) <= (uint32_t) n) r++;
+    return r;
+}
+
+// r_bins: block (ring, chunk) counts the pixels with ring * width <= r < (ring + 1) * width
+// over the planes of the chunk.  Eight lanes take a row: its pixels of the ring are at most
+// two x intervals (of about `width` each for most rows, hence eight), a lane per pixel, which
+// reads that pixel of every plane, eight ahead of their counting.  The outer, larger rings
+// start first.  Distances stay below 2^31 (the host checks).
+template <bool EXACT>
+__global__ void __launch_bounds__(1024) ring_histograms(const uint16_t *__restrict__ voxels, int64_t nzl, int Ny,
+                                                        int Nx, int y_start, int x_start, BinMap vm, int cy, int cx,
+                                                        int rings, int width, int64_t per,
+                                                        unsigned long long *__restrict__ r_bins, int voxel_bins,
+                                                        int n_r) {
+    extern __shared__ uint32_t counters[];
+    const int64_t chunks = (nzl + per - 1) / per;
+    const int ring = rings - 1 - (int) (blockIdx.x / chunks);
+    const int64_t z0 = blockIdx.x % chunks * per;
+    const int planes = (int) min(per, nzl - z0);
+    const int r0 = ring * width, r1 = min(r0 + width, n_r);
+    counters_clear(counters, (r1 - r0) * voxel_bins);
+    const int64_t plane = (int64_t) Ny * Nx;
+    const int inner = r0 * r0, outer = r1 * r1 - 1;  // squared distances inner .. outer
+    const int y_end = min(Ny - 1, cy + r1 - 1), lane = threadIdx.x & 7;
+    for (int y = max(y_start, cy - r1 + 1) + (threadIdx.x >> 3); y <= y_end; y += blockDim.x >> 3) {
+        const int dy2 = (y - cy) * (y - cy);
+        const int far = isqrt32(outer - dy2), near = dy2 >= inner ? 0 : isqrt32(inner - dy2 - 1) + 1;
+        // right: cx + near .. cx + far; left: cx - far .. cx - max(near, 1)
+        const int right = max(cx + near, x_start), n_right = max(0, min(cx + far, Nx - 1) - right + 1);
+        const int left = max(cx - far, x_start), n_left = max(0, min(cx - max(near, 1), Nx - 1) - left + 1);
+        const uint16_t *row = voxels + z0 * plane + (int64_t) y * Nx;
+        for (int k = lane; k < n_right + n_left; k += 8) {
+            const int x = k < n_right ? right + k : left + (k - n_right);
+            uint32_t *c = counters + (isqrt32(dy2 + (x - cx) * (x - cx)) - r0) * voxel_bins;
+            const uint16_t *p = row + x;
+            for (int z = 0; z < planes; z += 8, p += 8 * plane) {
+                int v[8];
+#pragma unroll
+                for (int j = 0; j < 8; j++) v[j] = z + j < planes ? __ldg(p + j * plane) : -1;
+#pragma unroll
+                for (int j = 0; j < 8; j++) {
+                    const int b = bin_of<EXACT>(vm, v[j]);
+                    if (b >= 0 && v[j] >= 0) atomicAdd(c + b, 1u);
+                }
+            }
+        }
+    }
+    counters_flush(counters, (r1 - r0) * voxel_bins, r_bins + (int64_t) r0 * voxel_bins);
 }
 
 // floor((bins - 1) * ((v - lo) / (hi - lo))) in FP64, as the reference writes it.
@@ -224,9 +367,13 @@ int64_t ref_bin(double v, double lo, double hi, int64_t bins) {
     return (int64_t) std::floor((double) u);
 }
 
-// Thresholds of an exact bin table (-1: not counted) whose counted values form one
-// contiguous range with bins non-decreasing in the value; checks the FP32 estimate.
-// `scale` and `origin` are the FP64 slope and zero of the bin expression.
+// The map of an exact bin table (-1: not counted) whose counted values form one contiguous
+// range with bins non-decreasing in the value.  `scale` and `origin` are the FP64 slope and
+// zero of the bin expression.  The fixed-point bin floor((d * slope + offset) / 2^32) is
+// evaluated here for every counted value, with the offset raised in steps until all of them
+// are right (values that fall on a bin's edge need it above the rounding of the slope); where
+// no offset is, which takes an expression whose own FP64 rounding is uneven, the thresholds
+// settle it, provided that the bin is within one.  Leaves T empty if they are not needed.
 int make_bin_map(const std::vector<int32_t> &tab, int64_t bins, double scale, double origin,
                  std::vector<uint32_t> &T, BinMap &m, const char *what) {
     int lo = -1, hi = -1;
@@ -235,12 +382,11 @@ int make_bin_map(const std::vector<int32_t> &tab, int64_t bins, double scale, do
             if (lo < 0) lo = v;
             hi = v;
         }
-    T.assign(bins + 1, 0);
+    T.clear();
+    m = BinMap{};
     m.bins = (int) bins;
     if (lo < 0) {  // nothing counted: a range no uint16 reaches
         m.lo = 65536 + 1;
-        m.span = 0;
-        m.a = m.c = 0.0f;
         return MAXI_OK;
     }
     for (int v = lo; v <= hi; v++)
@@ -248,18 +394,32 @@ int make_bin_map(const std::vector<int32_t> &tab, int64_t bins, double scale, do
             return set_error(MAXI_ERR_UNSUPPORTED, "%s bins are not monotone in the value", what);
     m.lo = lo;
     m.span = hi - lo;
-    m.a = (float) scale;
-    m.c = (float) (((double) lo - origin) * scale);
+    if (m.span == 0) {  // one counted value
+        m.offset = (uint64_t) tab[lo] << 32;
+        return MAXI_OK;
+    }
+    const double one = 4294967296.0;
+    const uint64_t slope = (uint64_t) std::llround(scale * one);  // scale < 2^20: two values are counted
+    m.mul_lo = (uint32_t) slope;
+    m.mul_hi = (uint32_t) (slope >> 32);
+    const double base = std::max(0.0, ((double) lo - origin) * scale);
+    auto bin = [&](int v) {
+        const uint64_t d = (uint64_t) (v - lo);
+        return (int64_t) ((d * m.mul_lo + m.offset) >> 32) + (int64_t) (uint32_t) (d * m.mul_hi);
+    };
+    int64_t off_by = 0;
+    for (int step = 0; step <= 20; step++) {
+        m.offset = (uint64_t) std::floor(base * one) + (uint64_t(1) << step);
+        off_by = 0;
+        for (int v = lo; v <= hi && off_by <= 1; v++) off_by = std::max(off_by, std::abs(bin(v) - (int64_t) tab[v]));
+        if (off_by == 0) return MAXI_OK;
+    }
+    if (off_by > 1) return set_error(MAXI_ERR_UNSUPPORTED, "%s bin estimate off by more than one", what);
+    T.assign(bins + 1, 0);
     int64_t b = 0;
     for (int v = lo; v <= hi; v++)
         while (b <= tab[v]) T[b++] = (uint32_t) v;
     while (b <= bins) T[b++] = (uint32_t) hi + 1;
-    for (int v = lo; v <= hi; v++) {
-        int est = (int) std::fmaf((float) (v - lo), m.a, m.c);
-        est = std::min(std::max(est, 0), m.bins - 1);
-        if (std::abs(est - tab[v]) > 1)
-            return set_error(MAXI_ERR_UNSUPPORTED, "%s bin estimate off by more than one at value %d", what, v);
-    }
     return MAXI_OK;
 }
 
@@ -326,6 +486,7 @@ struct DeviceTables {
 
 int upload(DeviceTables &t, cudaStream_t st) {
     const size_t bytes = t.host.size() * sizeof(uint32_t);
+    if (bytes == 0) return MAXI_OK;
     if (cudaMallocAsync(reinterpret_cast<void **>(&t.dev), bytes, st) != cudaSuccess) {
         cudaGetLastError();
         t.dev = nullptr;
@@ -343,6 +504,65 @@ int finish(DeviceTables &t, cudaStream_t st, int rc, const char *what) {
     if (rc != MAXI_OK) return rc;
     if (e == cudaSuccess) e = e2;
     return e == cudaSuccess ? MAXI_OK : set_cuda_error(e, what);
+}
+
+// Shared counters of one block of the strip and ring forms (128 KB).
+constexpr int kBlockCells = 32768;
+constexpr int kMaxSharedBins = 8192;
+// Voxels below which the direct form's single launch is the faster one.
+constexpr int64_t kAxisMinVoxels = int64_t(1) << 17;
+
+int axis_launches(const uint16_t *voxels, int64_t nzl, int64_t Ny, int Nx, int64_t z_start, int64_t y_start, int x_start,
+                  const BinMap &vm, int64_t cy, int64_t cx, unsigned long long *xb, unsigned long long *yb,
+                  unsigned long long *zb, unsigned long long *rb, int voxel_bins, int64_t n_r, bool vec,
+                  int64_t farthest, cudaStream_t st) {
+    const int64_t sms = sm_count(), rows = nzl * Ny;
+    if (voxel_bins > kMaxSharedBins || rows * Nx < kAxisMinVoxels || farthest >= (1 << 15) || n_r >= (1 << 15)) {
+        const unsigned grid = (unsigned) std::min<int64_t>(rows, sms * 16);
+        auto direct = vec ? axis_histograms_direct<true> : axis_histograms_direct<false>;
+        direct<<<grid, vec ? 128 : 256, 0, st>>>(voxels, nzl, Ny, Nx, z_start, y_start, x_start, vm, cy, cx, xb, yb, zb,
+                                                 rb, voxel_bins, n_r);
+        return MAXI_OK;
+    }
+    const bool exact = !vm.T;
+    auto launch = [&](auto kernel, int64_t grid, int threads, int cells, auto... args) {
+        const int smem = cells * (int) sizeof(uint32_t);
+        cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
+        if (e != cudaSuccess) return set_cuda_error(e, "axis histograms set-up");
+        kernel<<<(unsigned) grid, threads, smem, st>>>(args...);
+        return (int) MAXI_OK;
+    };
+    // z and y: several chunks per plane (or y) where there are few of them, of 16 rows at least.
+    auto row_sets = [&](int64_t sets, int64_t first_set, int64_t set_step, int64_t row_step, int64_t row_count,
+                        int64_t first_row, unsigned long long *bins) {
+        const int64_t n = row_count - first_row, counted = sets - first_set;
+        const int64_t chunks = std::max<int64_t>(1, std::min(ceil_div(sms * 8, counted), n / 16));
+        const int64_t per = ceil_div(n, chunks);
+        const RowSets s{sets, set_step, row_step, row_count, first_row, per, first_set, bins};
+        return launch(vec ? (exact ? row_set_histograms<true, true> : row_set_histograms<true, false>)
+                          : (exact ? row_set_histograms<false, true> : row_set_histograms<false, false>), counted * ceil_div(n, per), 256,
+                      voxel_bins, voxels, Nx, x_start, vm, s, voxel_bins);
+    };
+    int rc = row_sets(nzl, 0, Ny, 1, Ny, y_start, zb + z_start * voxel_bins);
+    if (rc == MAXI_OK) rc = row_sets(Ny, y_start, 1, Ny, nzl, 0, yb);
+    if (rc) return rc;
+    // x: strips of 8, or as many as the counters allow; chunks of at least 2048 rows.
+    const int strip = std::min(kVec, kBlockCells / voxel_bins), strips = (int) ceil_div(Nx, strip);
+    const int64_t x_chunks = std::max<int64_t>(1, std::min(ceil_div(sms * 4, strips), rows / 2048));
+    const int64_t x_per = ceil_div(rows, x_chunks);
+    const bool wide = vec && strip == kVec;
+    rc = launch(wide ? (exact ? strip_histograms<true, true> : strip_histograms<true, false>)
+                     : (exact ? strip_histograms<false, true> : strip_histograms<false, false>), strips * ceil_div(rows, x_per),
+                1024, strip * voxel_bins, voxels, rows, Ny, Nx, y_start, x_start, vm, strips, strip, x_per, xb, voxel_bins);
+    if (rc) return rc;
+    // r: rings of as many radii as the counters allow; 16 planes per block.
+    const int64_t radii = std::min<int64_t>(n_r, (int64_t) (1.4142136 * (double) farthest) + 2);
+    const int width = (int) std::min<int64_t>(radii, std::max(1, kBlockCells / voxel_bins));
+    const int rings = (int) ceil_div(radii, width);
+    const int64_t per = std::min<int64_t>(nzl, 16);
+    return launch(exact ? ring_histograms<true> : ring_histograms<false>, rings * ceil_div(nzl, per), 1024,
+                  width * voxel_bins, voxels, nzl, (int) Ny, Nx, (int) y_start, x_start, vm, (int) cy, (int) cx, rings,
+                  width, per, rb, voxel_bins, (int) n_r);
 }
 
 }  // namespace
@@ -394,8 +614,8 @@ extern "C" int maxi_field_histogram(const uint16_t *voxels, int64_t nZ, int64_t 
     const size_t o_x = t.add(xmap.data(), xmap.size());
     rc = upload(t, st);
     if (rc == MAXI_OK) {
-        vm.T = t.dev + o_vT;
-        fm.T = t.dev + o_fT;
+        if (!vT.empty()) vm.T = t.dev + o_vT;
+        if (!fT.empty()) fm.T = t.dev + o_fT;
         const int32_t *zm = reinterpret_cast<const int32_t *>(t.dev + o_z);
         const int32_t *ym = reinterpret_cast<const int32_t *>(t.dev + o_y);
         const int32_t *xm = reinterpret_cast<const int32_t *>(t.dev + o_x);
@@ -442,24 +662,12 @@ extern "C" int maxi_axis_histograms(const uint16_t *voxels, int64_t nz_block, in
     const size_t o_vT = t.add(vT.data(), vT.size());
     rc = upload(t, st);
     if (rc == MAXI_OK) {
-        vm.T = t.dev + o_vT;
+        if (!vT.empty()) vm.T = t.dev + o_vT;
         auto *xb = reinterpret_cast<unsigned long long *>(x_bins), *yb = reinterpret_cast<unsigned long long *>(y_bins);
         auto *zb = reinterpret_cast<unsigned long long *>(z_bins), *rb = reinterpret_cast<unsigned long long *>(r_bins);
         const bool vec = Nx % kVec == 0 && reinterpret_cast<uintptr_t>(voxels) % 16 == 0;
-        const int threads = vec ? 128 : 256;
-        // Row privatisation: 2 * voxel_bins + 1 words of shared memory, up to 8192 bins.
-        const bool priv = voxel_bins <= 8192;
-        const size_t smem = priv ? (2 * (size_t) voxel_bins + 1) * sizeof(uint32_t) : 0;
-        const unsigned grid = (unsigned) std::min<int64_t>(nzl * Ny, (int64_t) sm_count() * 16);
-        auto launch = [&](auto kern) {
-            cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int) smem);
-            if (e != cudaSuccess) return set_cuda_error(e, "axis histograms set-up");
-            kern<<<grid, threads, smem, st>>>(voxels, nzl, Ny, (int) Nx, z_start, y_start, (int) x_start, vm, cy, cx,
-                                              xb, yb, zb, rb, (int) voxel_bins, n_r);
-            return (int) MAXI_OK;
-        };
-        if (vec) rc = priv ? launch(axis_histograms_kernel<true, true>) : launch(axis_histograms_kernel<true, false>);
-        else rc = priv ? launch(axis_histograms_kernel<false, true>) : launch(axis_histograms_kernel<false, false>);
+        rc = axis_launches(voxels, nzl, Ny, (int) Nx, z_start, y_start, (int) x_start, vm, cy, cx, xb, yb, zb, rb,
+                           (int) voxel_bins, n_r, vec, std::max(rx, ry), st);
     }
     return finish(t, st, rc, "axis histograms");
 }
