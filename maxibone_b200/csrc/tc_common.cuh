@@ -318,6 +318,15 @@ template <> struct Pair16<__nv_bfloat16> {
     static __device__ __forceinline__ float2 widen(uint32_t q) {
         return make_float2(__uint_as_float(q << 16), __uint_as_float(q & 0xffff0000u));
     }
+    // w - q, exactly: a mixed-precision FMA per value (q x -1 + w) reads the 16-bit halves as
+    // they are, without the shift and the mask that widen() takes on the ALU pipe.
+    static __device__ __forceinline__ float2 residual(uint32_t q, float2 w) {
+        float2 c;
+        asm("{\n.reg .b16 lo, hi;\nmov.b32 {lo, hi}, %2;\n"
+            "fma.rn.f32.bf16 %0, lo, %5, %3;\nfma.rn.f32.bf16 %1, hi, %5, %4;\n}"
+            : "=f"(c.x), "=f"(c.y) : "r"(q), "f"(w.x), "f"(w.y), "h"((uint16_t) 0xBF80));
+        return c;
+    }
 };
 template <> struct Pair16<__half> {
     static __device__ __forceinline__ uint32_t cvt(float lo, float hi) {
@@ -326,6 +335,13 @@ template <> struct Pair16<__half> {
     }
     static __device__ __forceinline__ float2 widen(uint32_t q) {
         return __half22float2(*reinterpret_cast<const __half2 *>(&q));
+    }
+    static __device__ __forceinline__ float2 residual(uint32_t q, float2 w) {
+        float2 c;
+        asm("{\n.reg .b16 lo, hi;\nmov.b32 {lo, hi}, %2;\n"
+            "fma.rn.f32.f16 %0, lo, %5, %3;\nfma.rn.f32.f16 %1, hi, %5, %4;\n}"
+            : "=f"(c.x), "=f"(c.y) : "r"(q), "f"(w.x), "f"(w.y), "h"((uint16_t) 0xBC00));
+        return c;
     }
 };
 
@@ -342,7 +358,7 @@ template <typename S, bool MASKED>
 __device__ __forceinline__ void narrow32_pairs(const float (&a)[32], float scale, bool ef, uint32_t force1,
                                                uint32_t live, uint32_t (&d)[16]) {
     float2 c = make_float2(0.0f, 0.0f);
-    const float2 s2 = make_float2(scale, scale), m1 = make_float2(-1.0f, -1.0f);
+    const float2 s2 = make_float2(scale, scale);
 #pragma unroll
     for (int j = 0; j < 16; j++) {
         const float2 v = make_float2(a[j], a[16 + j]);
@@ -354,7 +370,7 @@ __device__ __forceinline__ void narrow32_pairs(const float (&a)[32], float scale
             if ((force1 >> (16 + j)) & 1u) w.y = 1.0f;
         }
         const uint32_t q = Pair16<S>::cvt(w.x, w.y);
-        if (ef) c = __ffma2_rn(Pair16<S>::widen(q), m1, w);
+        if (ef) c = Pair16<S>::residual(q, w);
         d[j] = q;
     }
 }
@@ -366,7 +382,7 @@ template <typename S>
 __device__ __forceinline__ void narrow64_pairs_forced(const float (&a)[64], float scale, bool ef, uint32_t f0,
                                                       uint32_t f1, uint32_t (&d0)[16], uint32_t (&d1)[16]) {
     float2 c0 = make_float2(0.0f, 0.0f), c1 = make_float2(0.0f, 0.0f);
-    const float2 s2 = make_float2(scale, scale), m1 = make_float2(-1.0f, -1.0f);
+    const float2 s2 = make_float2(scale, scale);
 #pragma unroll
     for (int j = 0; j < 16; j++) {
         const float2 v0 = make_float2(a[j], a[16 + j]), v1 = make_float2(a[32 + j], a[48 + j]);
@@ -378,8 +394,8 @@ __device__ __forceinline__ void narrow64_pairs_forced(const float (&a)[64], floa
         if ((f1 >> (16 + j)) & 1u) w1.y = 1.0f;
         const uint32_t q0 = Pair16<S>::cvt(w0.x, w0.y), q1 = Pair16<S>::cvt(w1.x, w1.y);
         if (ef) {
-            c0 = __ffma2_rn(Pair16<S>::widen(q0), m1, w0);
-            c1 = __ffma2_rn(Pair16<S>::widen(q1), m1, w1);
+            c0 = Pair16<S>::residual(q0, w0);
+            c1 = Pair16<S>::residual(q1, w1);
         }
         d0[j] = q0;
         d1[j] = q1;
@@ -394,7 +410,7 @@ template <typename S>
 __device__ __forceinline__ void narrow64_pairs_forced_adjacent(const float (&a)[64], float scale, bool ef, uint32_t f0,
                                                                uint32_t f1, uint32_t (&d0)[16], uint32_t (&d1)[16]) {
     float2 c0 = make_float2(0.0f, 0.0f), c1 = make_float2(0.0f, 0.0f);
-    const float2 s2 = make_float2(scale, scale), m1 = make_float2(-1.0f, -1.0f);
+    const float2 s2 = make_float2(scale, scale);
 #pragma unroll
     for (int j = 0; j < 16; j++) {
         const float2 v0 = make_float2(a[2 * j], a[2 * j + 1]), v1 = make_float2(a[32 + 2 * j], a[33 + 2 * j]);
@@ -406,8 +422,8 @@ __device__ __forceinline__ void narrow64_pairs_forced_adjacent(const float (&a)[
         if ((f1 >> (16 + j)) & 1u) w1.y = 1.0f;
         const uint32_t q0 = Pair16<S>::cvt(w0.x, w0.y), q1 = Pair16<S>::cvt(w1.x, w1.y);
         if (ef) {
-            c0 = __ffma2_rn(Pair16<S>::widen(q0), m1, w0);
-            c1 = __ffma2_rn(Pair16<S>::widen(q1), m1, w1);
+            c0 = Pair16<S>::residual(q0, w0);
+            c1 = Pair16<S>::residual(q1, w1);
         }
         d0[j] = q0;
         d1[j] = q1;
@@ -425,7 +441,7 @@ __device__ __forceinline__ void narrow64_pairs_forced_adjacent(const float (&a)[
 template <typename S>
 __device__ __forceinline__ void narrow32_quads(const float (&a)[32], float scale, bool ef, uint32_t (&d)[16]) {
     float2 c0 = make_float2(0.0f, 0.0f), c1 = make_float2(0.0f, 0.0f);
-    const float2 s2 = make_float2(scale, scale), m1 = make_float2(-1.0f, -1.0f);
+    const float2 s2 = make_float2(scale, scale);
 #pragma unroll
     for (int j = 0; j < 8; j++) {
         float2 w0 = make_float2(a[j], a[8 + j]), w1 = make_float2(a[16 + j], a[24 + j]);
@@ -433,8 +449,8 @@ __device__ __forceinline__ void narrow32_quads(const float (&a)[32], float scale
         w1 = ef ? __ffma2_rn(w1, s2, c1) : __fmul2_rn(w1, s2);
         const uint32_t q0 = Pair16<S>::cvt(w0.x, w0.y), q1 = Pair16<S>::cvt(w1.x, w1.y);
         if (ef) {
-            c0 = __ffma2_rn(Pair16<S>::widen(q0), m1, w0);
-            c1 = __ffma2_rn(Pair16<S>::widen(q1), m1, w1);
+            c0 = Pair16<S>::residual(q0, w0);
+            c1 = Pair16<S>::residual(q1, w1);
         }
         d[j] = q0;
         d[8 + j] = q1;
@@ -447,7 +463,7 @@ template <typename S>
 __device__ __forceinline__ void narrow64_quads(const float (&a)[64], float scale, bool ef, uint32_t (&d0)[16],
                                                uint32_t (&d1)[16]) {
     float2 c[4] = {make_float2(0.0f, 0.0f), make_float2(0.0f, 0.0f), make_float2(0.0f, 0.0f), make_float2(0.0f, 0.0f)};
-    const float2 s2 = make_float2(scale, scale), m1 = make_float2(-1.0f, -1.0f);
+    const float2 s2 = make_float2(scale, scale);
 #pragma unroll
     for (int j = 0; j < 8; j++) {
 #pragma unroll
@@ -456,7 +472,7 @@ __device__ __forceinline__ void narrow64_quads(const float (&a)[64], float scale
             float2 w = make_float2(a[b + j], a[b + 8 + j]);
             w = ef ? __ffma2_rn(w, s2, c[h]) : __fmul2_rn(w, s2);
             const uint32_t q = Pair16<S>::cvt(w.x, w.y);
-            if (ef) c[h] = __ffma2_rn(Pair16<S>::widen(q), m1, w);
+            if (ef) c[h] = Pair16<S>::residual(q, w);
             ((h >> 1) ? d1 : d0)[8 * (h & 1) + j] = q;
         }
     }
