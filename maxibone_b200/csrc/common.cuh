@@ -163,11 +163,12 @@ template <> __device__ __forceinline__ uint32_t mask32<MAXI_MASK_BITPACKED>(cons
 }
 
 // Quantisation of the reference (src/lib/cpp/cpu/diffusion.cc:191-195):
-// floor(v * 65535.0f) in FP32, clamped to the uint16 range.
+// floor(v * 65535.0f) in FP32, clamped to the uint16 range (0 for a NaN).  The clamp is taken
+// on v; adding 2^23 with rounding down leaves the floor in the sum's low bits, without the
+// floor and conversion instructions of the quarter-rate pipe (two per voxel, which bound
+// the last repetition's pass: 1024^3 BF16 fused 2.16 ms against 1.14 of the others).
 __device__ __forceinline__ uint16_t quantise_u16(float v) {
-    float q = floorf(v * 65535.0f);
-    q = fminf(fmaxf(q, 0.0f), 65535.0f);
-    return (uint16_t) q;
+    return (uint16_t) __float_as_uint(__fadd_rd(__saturatef(v) * 65535.0f, 8388608.0f));
 }
 __device__ __forceinline__ uint16_t quantise_u16(double v) {
     double q = floor(v * 65535.0);
