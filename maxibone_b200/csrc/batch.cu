@@ -176,8 +176,7 @@ static cudaError_t enqueue_init(maxi_batch_plan *p, const std::vector<int> &idx,
     for (int i : idx) {
         BatchVolume &bv = p->vols[i];
         const int64_t n = bv.v.nz * bv.v.ny * bv.v.nx;
-        cudaError_t e = launch_bitpack_encode(static_cast<const uint8_t *>(bv.v.mask), n, vol_packed(p, bv), false, st);
-        if (e == cudaSuccess) e = launch_init_field<S>(vol_packed(p, bv), MAXI_MASK_BITPACKED, vol_buf<S>(p, bv, 0), n, st);
+        cudaError_t e = launch_init_field<S>(bv.v.mask, MAXI_MASK_U8, vol_packed(p, bv), vol_buf<S>(p, bv, 0), n, st);
         if (e != cudaSuccess) return e;
     }
     return cudaSuccess;
@@ -190,7 +189,12 @@ template <typename S>
 static cudaError_t enqueue_single(maxi_batch_plan *p, BatchVolume &bv, int32_t extra_flags, cudaStream_t st,
                                   bool fused = false) {
     const int64_t n = bv.v.nz * bv.v.ny * bv.v.nx;
-    cudaError_t e = launch_bitpack_encode(static_cast<const uint8_t *>(bv.v.mask), n, vol_packed(p, bv), false, st);
+    // (The FP32 form's first pass reads the packed mask: no field to write.)
+    RunOpts o;
+    o.field_ready = sizeof(S) == 2;
+    cudaError_t e = o.field_ready
+                        ? launch_init_field<S>(bv.v.mask, MAXI_MASK_U8, vol_packed(p, bv), vol_buf<S>(p, bv, 0), n, st)
+                        : launch_bitpack_encode(static_cast<const uint8_t *>(bv.v.mask), n, vol_packed(p, bv), false, st);
     if (e != cudaSuccess) return e;
     const Volume vol{bv.v.nz, bv.v.ny, bv.v.nx};
     // The batched tensor-core launches run the y and x passes as separate
@@ -199,7 +203,7 @@ static cudaError_t enqueue_single(maxi_batch_plan *p, BatchVolume &bv, int32_t e
     return dispatch_unrolled<S>(vol, vol_packed(p, bv), MAXI_MASK_BITPACKED, bv.kernel.data(),
                                 (int) (bv.v.kernel_size / 2), bv.v.repititions, vol_buf<S>(p, bv, 0),
                                 vol_buf<S>(p, bv, 1), bv.v.output, bv.v.field_out,
-                                p->flags | extra_flags | (fused ? 0 : MAXI_FLAG_SEPARATE_PASSES), st);
+                                p->flags | extra_flags | (fused ? 0 : MAXI_FLAG_SEPARATE_PASSES), st, o);
 }
 
 // All repetitions of a tensor-core group as batched launches.

@@ -124,10 +124,16 @@ static cudaError_t run_typed(const Volume &v, const void *mask, int mask_fmt, co
         return run_generic<S, false>(v, mask, mask_fmt, kernel, radius, reps, b0, b1, out_u16, field_out, o, st);
     }
     if constexpr (!is_f64) {
+        RunOpts opts = o;
         uint32_t *packed = reinterpret_cast<uint32_t *>(ws + 2 * round_up((int64_t) sizeof(S) * v.n(), 256));
         if (mask_fmt == MAXI_MASK_U8) {
-            // Read the mask as 1 bit per voxel in every x pass: pack it once.
-            cudaError_t e = launch_bitpack_encode(static_cast<const uint8_t *>(mask), v.n(), packed, false, st);
+            // Read the mask as 1 bit per voxel in every x pass: pack it once, and write a
+            // 16-bit field's start with it (the FP32 form's first pass reads the packed mask).
+            opts.field_ready = sizeof(S) == 2 && !o.init_field;
+            ProfScope ps(MAXI_KERNEL_INIT, st);
+            cudaError_t e = opts.field_ready
+                                ? launch_init_field<S>(mask, MAXI_MASK_U8, packed, b0, v.n(), st)
+                                : launch_bitpack_encode(static_cast<const uint8_t *>(mask), v.n(), packed, false, st);
             if (e != cudaSuccess) return e;
             mask = packed;
             mask_fmt = MAXI_MASK_BITPACKED;
@@ -138,7 +144,7 @@ static cudaError_t run_typed(const Volume &v, const void *mask, int mask_fmt, co
             mask = packed;
         }
         return dispatch_unrolled<S>(v, mask, mask_fmt, kernel, radius, reps, b0, b1, out_u16,
-                                    static_cast<float *>(field_out), flags, st, o);
+                                    static_cast<float *>(field_out), flags, st, opts);
     }
     return cudaErrorInvalidValue;
 }

@@ -8,7 +8,7 @@ namespace maxi {
 
 int radius_bucket(int r) { return radius_bucket_impl(r); }
 
-template cudaError_t launch_init_field<float>(const void *, int, float *, int64_t, cudaStream_t);
+template cudaError_t launch_init_field<float>(const void *, int, uint32_t *, float *, int64_t, cudaStream_t);
 
 namespace {
 
@@ -117,7 +117,7 @@ cudaError_t dispatch_unrolled<float>(const Volume &v, const void *mask, int mask
         ProfScope ps(MAXI_KERNEL_INIT, st);
         if (o.init_field)
             field_from_f32<float><<<std::min<int64_t>(ceil_div(v.n(), 256), 148 * 64), 256, 0, st>>>(o.init_field, buf0, v.n());
-        else if ((e = launch_init_field<float>(mask, mask_fmt, buf0, v.n(), st)) != cudaSuccess)
+        else if ((e = launch_init_field<float>(mask, mask_fmt, nullptr, buf0, v.n(), st)) != cudaSuccess)
             return e;
     }
     if (reps > 0) note_path(MAXI_PATH_CUDA_CORES);

@@ -16,9 +16,10 @@ struct Volume {
 // the reference encode's `mask & 1`; otherwise the diffusion's `mask > 0`.
 cudaError_t launch_bitpack_encode(const uint8_t *mask, int64_t n, uint32_t *packed, bool keep_bit0, cudaStream_t st);
 
-// field <- mask > 0 ? 1 : 0 in the storage type (rep-0 input).
+// field <- mask > 0 ? 1 : 0 in the storage type (rep-0 input); from a uint8 mask also its
+// bit-packed copy, unless `packed` is NULL.
 template <typename S>
-cudaError_t launch_init_field(const void *mask, int mask_fmt, S *field, int64_t n, cudaStream_t st);
+cudaError_t launch_init_field(const void *mask, int mask_fmt, uint32_t *packed, S *field, int64_t n, cudaStream_t st);
 
 // Smallest radius with an unrolled instantiation that is >= r, or -1.
 int radius_bucket(int r);
@@ -32,6 +33,8 @@ struct RunOpts {
     // Start from this FP32 field (device or mapped host memory, nz*ny*nx
     // values) instead of the mask (out-of-core exchange rounds).
     const float *init_field = nullptr;
+    // The first buffer already holds the initial field (launch_init_field).
+    bool field_ready = false;
     // The last repetition waits for this event before it starts (lets the
     // caller overlap a copy out of the output buffers with the earlier ones).
     cudaEvent_t final_wait = nullptr;

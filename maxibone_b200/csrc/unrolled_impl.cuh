@@ -37,6 +37,21 @@ static cudaError_t set_smem(F *f, int bytes) {
     return cudaFuncSetAttribute(f, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes);
 }
 
+template <typename S>
+cudaError_t launch_init_field(const void *mask, int mask_fmt, uint32_t *packed, S *field, int64_t n, cudaStream_t st) {
+    const int64_t blocks = std::min<int64_t>(ceil_div(n, 256 * 8), 148 * 32);
+    if (mask_fmt == MAXI_MASK_BITPACKED) {
+        init_from_mask<S, MAXI_MASK_BITPACKED><<<blocks, 256, 0, st>>>(mask, nullptr, field, n);
+    } else if (reinterpret_cast<uintptr_t>(mask) % 8 == 0) {
+        init_from_mask<S, MAXI_MASK_U8><<<blocks, 256, 0, st>>>(mask, packed, field, n);
+    } else {  // a mask at an odd address: a voxel per thread
+        mask_to_field<S, MAXI_MASK_U8, false><<<std::min<int64_t>(ceil_div(n, 256), 148 * 64), 256, 0, st>>>(
+            mask, field, nullptr, nullptr, n);
+        if (packed) return launch_bitpack_encode(static_cast<const uint8_t *>(mask), n, packed, false, st);
+    }
+    return cudaGetLastError();
+}
+
 // One repetition loop for bucket radius R.  EF: error-feedback rounding of the
 // 16-bit storage type (see passes.cuh); use_tc: z and y passes on the tensor
 // cores (tc_pass.cu).
@@ -62,16 +77,12 @@ static cudaError_t run_unrolled(const Volume &v, const void *mask, int mask_fmt,
     auto *xfinal = mask_fmt == MAXI_MASK_U8 ? xu8f : xbpf;
 
     const int64_t n = v.n();
-    {
-        const int threads = 256;
-        const int64_t blocks = std::min<int64_t>((n + threads - 1) / threads, 148 * 64);
+    if (!o.field_ready) {
         ProfScope ps(MAXI_KERNEL_INIT, st);
         if (o.init_field)
-            field_from_f32<S><<<blocks, threads, 0, st>>>(o.init_field, buf0, n);
-        else if (mask_fmt == MAXI_MASK_U8)
-            mask_to_field<S, MAXI_MASK_U8, false><<<blocks, threads, 0, st>>>(mask, buf0, nullptr, nullptr, n);
-        else
-            mask_to_field<S, MAXI_MASK_BITPACKED, false><<<blocks, threads, 0, st>>>(mask, buf0, nullptr, nullptr, n);
+            field_from_f32<S><<<std::min<int64_t>(ceil_div(n, 256), 148 * 64), 256, 0, st>>>(o.init_field, buf0, n);
+        else if ((e = launch_init_field<S>(mask, mask_fmt, nullptr, buf0, n, st)) != cudaSuccess)
+            return e;
     }
     const int64_t plane = v.ny * v.nx;
     // Tensor-core x pass: vector epilogue needs 16-byte aligned mask (u8), output and field.
@@ -147,16 +158,6 @@ static cudaError_t run_unrolled(const Volume &v, const void *mask, int mask_fmt,
         if (e != cudaSuccess) return e;
         if (!last) std::swap(buf0, buf1);
     }
-    return cudaGetLastError();
-}
-
-template <typename S>
-cudaError_t launch_init_field(const void *mask, int mask_fmt, S *field, int64_t n, cudaStream_t st) {
-    const int64_t blocks = std::min<int64_t>(ceil_div(n, 256), 148 * 64);
-    if (mask_fmt == MAXI_MASK_U8)
-        mask_to_field<S, MAXI_MASK_U8, false><<<blocks, 256, 0, st>>>(mask, field, nullptr, nullptr, n);
-    else
-        mask_to_field<S, MAXI_MASK_BITPACKED, false><<<blocks, 256, 0, st>>>(mask, field, nullptr, nullptr, n);
     return cudaGetLastError();
 }
 
