@@ -402,9 +402,9 @@ int maxi_diffusion_in_memory(const uint8_t *voxels, int64_t nz, int64_t ny, int6
     uint8_t *d_mask = reinterpret_cast<uint8_t *>(base + mask_off);
     uint16_t *d_out = reinterpret_cast<uint16_t *>(base + out_off);
     cudaStream_t st = cache->stream;
-    // Pageable caller buffers of some size go through pinned staging with
-    // several host threads; pinned ones are copied directly.
-    const int64_t stage_min = int64_t(64) << 20;
+    // Pageable caller buffers from 4 MB on go through pinned staging with several host threads
+    // (below, one driver-staged copy is as fast); pinned ones are copied directly.
+    const int64_t stage_min = int64_t(4) << 20;
     const bool stage_in = n >= stage_min && host_pageable(voxels);
     const bool stage_out = 2 * n >= stage_min && host_pageable(output);
     cudaError_t e = stage_in ? copy_to_device_staged(d_mask, voxels, n, st)
@@ -437,6 +437,7 @@ int maxi_release_cached_memory(void) {
     clear_error();
     release_device_caches();
     release_morphology_scratch();
+    release_staging_buffers();
     return MAXI_OK;
 }
 
