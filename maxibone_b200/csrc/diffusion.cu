@@ -19,6 +19,7 @@
 #include "host_copy.h"
 #include "unrolled.h"
 #include "profiler.h"
+#include "scratch.h"
 #include "tc_pass.h"
 #include "tc_batch.h"
 
@@ -436,7 +437,7 @@ int maxi_keep_device_buffers(int keep) {
 int maxi_release_cached_memory(void) {
     clear_error();
     release_device_caches();
-    release_morphology_scratch();
+    release_scratch();
     release_staging_buffers();
     return MAXI_OK;
 }

@@ -14,157 +14,258 @@
 // the extremes the later steps need follow from the extremes of c over all
 // voxels and over the voxels inside the cylinder: two reduction passes (the
 // field maxima, then those extremes) and one conversion pass, each a read of
-// both fields -- HBM-bound.  The host does the scalar steps in FP32 between
-// the passes.  The cylinder is convex along x for every row, so each row's
+// both fields -- HBM-bound: 14 bytes per voxel.  The scalar steps between the passes are
+// done by every thread of the next pass, in FP32 in numpy's order, so the host reads back
+// once, at the end.  The cylinder is convex along x for every row, so each row's
 // inside voxels are one x interval, found on the host with numpy's own FP64
 // arithmetic (linspace(-1, 1, n)[i] = i * (2 / (n - 1)) - 1, last point 1).
+//
+// Divisions.  Two per voxel of the second pass and four of the third, all by per-call
+// scalars, bound those passes as divide sequences (803 and 1205 us at 384 x 1000 x 1000,
+// against 376 for the maxima).  They are done with the scalar's correctly rounded
+// reciprocal y instead: q = a y, then q + (a - q b) y with two FMAs, which is the
+// correctly rounded quotient (P. Markstein, Computation of elementary functions on the
+// IBM RISC System/6000 processor, IBM J. Res. Dev. 34, 1990, theorem 8.2) away from
+// over- and underflow; scalars that could bring one about keep the division.  Conversions
+// between uint16 and FP32 go through the bits of 2^23 + v rather than the quarter-rate
+// conversion instructions.
+// Every integer quotient of two uint16 values was compared with the division, and 2^31
+// random ones: all equal.
+// 384 x 1000 x 1000 on a B200, before and now: maxima 376 and 222 us (6.9 TB/s from DRAM and
+// L2), extremes 803 and 276, conversion 1205 and 385 (6.0 TB/s).
 #include <cmath>
+#include <type_traits>
 #include <vector>
 
 #include "common.cuh"
 #include "host_util.h"
+#include "scratch.h"
 
 namespace maxi {
 namespace {
 
+// All-zero to start with: minima are kept as maxima of the complemented keys.
 struct CombineStats {
-    unsigned int gmax, emax;        // field maxima
-    unsigned int cmin, cmax;        // extremes of c over all voxels (order-preserving keys)
-    unsigned int cmin_in, cmax_in;  // the same inside the cylinder
+    unsigned int gmax, emax;          // field maxima
+    unsigned int ncmin, cmax;         // extremes of c over all voxels (order-preserving keys)
+    unsigned int ncmin_in, cmax_in;   // the same inside the cylinder
     unsigned int pad[2];
 };
 
-// Float <-> unsigned key with the same order (for atomicMin / atomicMax).
+// Float <-> unsigned key with the same order (for atomicMax).
 __device__ __forceinline__ unsigned int fkey(float f) {
     const unsigned int u = __float_as_uint(f);
     return (u & 0x80000000u) ? ~u : (u | 0x80000000u);
 }
-float key_float(unsigned int k) {
-    const unsigned int u = (k & 0x80000000u) ? (k & 0x7fffffffu) : ~k;
-    float f;
-    memcpy(&f, &u, 4);
-    return f;
+__device__ __forceinline__ float key_float(unsigned int k) {
+    return __uint_as_float((k & 0x80000000u) ? (k & 0x7fffffffu) : ~k);
 }
 
-// The voxel loop over the flat volume, 8 voxels per step (16-byte loads) when
-// rows allow it, else 1; f(row, x, count) with the step's voxels inside one row.
-// f(row, y, x, count).  Chunk and row indices stay below 2^32 (the host checks),
-// so the index divisions are 32-bit.
-template <typename F>
-__device__ __forceinline__ void for_chunks(int64_t rows, int64_t ny, int64_t nx, bool vec, F &&f) {
-    const uint32_t step = vec ? 8u : 1u;
-    const uint32_t per_row = (uint32_t) (nx / step), yn = (uint32_t) ny;
-    const uint32_t total = (uint32_t) (rows * per_row);
-    for (uint32_t c = blockIdx.x * blockDim.x + threadIdx.x; c < total; c += gridDim.x * blockDim.x) {
-        const uint32_t row = c / per_row;
-        const uint32_t y = row % yn;
-        f((int64_t) row, (int) y, (int64_t) (c - row * per_row) * step, (int) step);
+// Correctly rounded division by a scalar (see the top of the file).
+struct Divisor {
+    float b, y;
+    bool plain;  // over- or underflow possible: divide
+    template <bool PLAIN = false>
+    __device__ __forceinline__ float2 quotient(float2 a) const {
+        if (PLAIN) return make_float2(__fdiv_rn(a.x, b), __fdiv_rn(a.y, b));
+        const float2 yy = make_float2(y, y), q = __fmul2_rn(a, yy);
+        return __ffma2_rn(__ffma2_rn(q, make_float2(-b, -b), a), yy, q);
     }
+};
+__device__ __forceinline__ Divisor divisor(float b) {
+    return {b, __fdiv_rn(1.0f, b), !(b >= 0x1p-60f && b <= 0x1p60f)};
+}
+// c = G / gm - E / em, in numpy's FP32 operations.
+__device__ __forceinline__ float2 combined(const Divisor &by_g, const Divisor &by_e, float2 g, float2 e) {
+    return __ffma2_rn(by_e.quotient(e), make_float2(-1.0f, -1.0f), by_g.quotient(g));
 }
 
-__device__ __forceinline__ void load8(const uint16_t *p, int cnt, float (&v)[8]) {
-    if (cnt == 8) {
-        const uint4 w = __ldg(reinterpret_cast<const uint4 *>(p));
-        const uint32_t a[4] = {w.x, w.y, w.z, w.w};
-#pragma unroll
-        for (int i = 0; i < 4; i++) {
-            v[2 * i] = (float) (a[i] & 0xffffu);
-            v[2 * i + 1] = (float) (a[i] >> 16);
-        }
-    } else {
-        v[0] = (float) __ldg(p);
-    }
+// Both halves of w as floats.
+__device__ __forceinline__ float2 halves(uint32_t w) {
+    const float2 v = make_float2(__uint_as_float(__byte_perm(w, 0x4b000000u, 0x7610)),
+                                 __uint_as_float(__byte_perm(w, 0x4b000000u, 0x7632)));
+    return __fadd2_rn(v, make_float2(-8388608.0f, -8388608.0f));
 }
 
-__device__ __forceinline__ unsigned int warp_max(unsigned int v) { return __reduce_max_sync(0xffffffffu, v); }
-__device__ __forceinline__ unsigned int warp_min(unsigned int v) { return __reduce_min_sync(0xffffffffu, v); }
-
-__global__ void field_maxima(const uint16_t *__restrict__ g, const uint16_t *__restrict__ e, int64_t rows, int64_t ny,
-                             int64_t nx, bool vec, CombineStats *st) {
+// The maxima of both fields over the flat volume, in packed 16-bit lanes.
+__global__ void __launch_bounds__(256) field_maxima(const uint16_t *__restrict__ g, const uint16_t *__restrict__ e,
+                                                    int64_t n, bool vec, CombineStats *st) {
+    const int64_t stride = (int64_t) gridDim.x * blockDim.x, thread = (int64_t) blockIdx.x * blockDim.x + threadIdx.x;
     unsigned int gm = 0, em = 0;
-    for_chunks(rows, ny, nx, vec, [&](int64_t row, int y, int64_t x, int cnt) {
-        float a[8], b[8];
-        load8(g + row * nx + x, cnt, a);
-        load8(e + row * nx + x, cnt, b);
-        for (int i = 0; i < cnt; i++) {
-            gm = max(gm, (unsigned int) a[i]);
-            em = max(em, (unsigned int) b[i]);
+    int64_t done = 0;
+    if (vec) {
+        constexpr int kAtOnce = 4;
+        const uint4 *gp = reinterpret_cast<const uint4 *>(g), *ep = reinterpret_cast<const uint4 *>(e);
+        const int64_t groups = n / 8;
+        for (int64_t i = (int64_t) blockIdx.x * kAtOnce * blockDim.x + threadIdx.x; i < groups; i += kAtOnce * stride) {
+            uint4 a[kAtOnce], b[kAtOnce];
+#pragma unroll
+            for (int k = 0; k < kAtOnce; k++) {
+                const int64_t j = min(i + k * blockDim.x, groups - 1);  // past the end: the last group again
+                a[k] = __ldg(gp + j), b[k] = __ldg(ep + j);
+            }
+#pragma unroll
+            for (int k = 0; k < kAtOnce; k++) {
+                gm = __vmaxu2(gm, __vmaxu2(__vmaxu2(a[k].x, a[k].y), __vmaxu2(a[k].z, a[k].w)));
+                em = __vmaxu2(em, __vmaxu2(__vmaxu2(b[k].x, b[k].y), __vmaxu2(b[k].z, b[k].w)));
+            }
         }
-    });
-    gm = warp_max(gm);
-    em = warp_max(em);
+        done = groups * 8;
+    }
+    for (int64_t i = done + thread; i < n; i += stride) {
+        gm = __vmaxu2(gm, __ldg(g + i));
+        em = __vmaxu2(em, __ldg(e + i));
+    }
+    gm = __reduce_max_sync(0xffffffffu, max(gm >> 16, gm & 0xffffu));
+    em = __reduce_max_sync(0xffffffffu, max(em >> 16, em & 0xffffu));
     if ((threadIdx.x & 31) == 0) {
         atomicMax(&st->gmax, gm);
         atomicMax(&st->emax, em);
     }
 }
 
-// c = G / gm - E / em with numpy's FP32 operations (no contraction).
-__device__ __forceinline__ float combined(float g, float e, float gm, float em) {
-    return __fsub_rn(__fdiv_rn(g, gm), __fdiv_rn(e, em));
-}
-
-__global__ void combined_extremes(const uint16_t *__restrict__ g, const uint16_t *__restrict__ e, int64_t rows,
-                                  int64_t ny, int64_t nx, bool vec, const int2 *__restrict__ inside, float gm, float em,
-                                  CombineStats *st) {
-    unsigned int lo = 0xffffffffu, hi = 0, lo_in = 0xffffffffu, hi_in = 0;
-    for_chunks(rows, ny, nx, vec, [&](int64_t row, int y, int64_t x, int cnt) {
-        const int2 iv = __ldg(inside + y);
-        float a[8], b[8];
-        load8(g + row * nx + x, cnt, a);
-        load8(e + row * nx + x, cnt, b);
-        for (int i = 0; i < cnt; i++) {
-            const unsigned int k = fkey(combined(a[i], b[i], gm, em));
-            lo = min(lo, k);
-            hi = max(hi, k);
-            if (x + i >= iv.x && x + i < iv.y) {
-                lo_in = min(lo_in, k);
-                hi_in = max(hi_in, k);
+// The walk of the other two passes: `lanes` (a power of two) threads per row, 8 voxels each
+// at a time (VEC: rows are 16-byte aligned) or one; row(r) for every row, then
+// voxels(r, x, a, b) with the two fields' voxels from x on.  Row indices stay below
+// 2^32 (the host checks), so their division is 32-bit.
+template <bool VEC, typename Row, typename Voxels>
+__device__ __forceinline__ void for_rows(const uint16_t *__restrict__ g, const uint16_t *__restrict__ e, int64_t rows,
+                                         int nx, int lanes, Row &&row, Voxels &&voxels) {
+    constexpr int V = VEC ? 8 : 1, kAtOnce = VEC ? 2 : 4;
+    const int lane = threadIdx.x & (lanes - 1);
+    const int64_t first = ((int64_t) blockIdx.x * blockDim.x + threadIdx.x) / lanes;
+    const int64_t step = (int64_t) gridDim.x * blockDim.x / lanes;
+    for (int64_t r = first; r < rows; r += step) {
+        row(r);
+        const uint16_t *gr = g + r * nx, *er = e + r * nx;
+        for (int x0 = lane * V; x0 < nx; x0 += kAtOnce * lanes * V) {
+            uint4 a[kAtOnce], b[kAtOnce];
+#pragma unroll
+            for (int k = 0; k < kAtOnce; k++) {
+                const int x = x0 + k * lanes * V;
+                if (x < nx) {
+                    if (VEC) {
+                        a[k] = __ldg(reinterpret_cast<const uint4 *>(gr + x));
+                        b[k] = __ldg(reinterpret_cast<const uint4 *>(er + x));
+                    } else {
+                        a[k].x = __ldg(gr + x);
+                        b[k].x = __ldg(er + x);
+                    }
+                }
+            }
+#pragma unroll
+            for (int k = 0; k < kAtOnce; k++) {
+                const int x = x0 + k * lanes * V;
+                if (x < nx) voxels(r, x, a[k], b[k]);
             }
         }
-    });
-    lo = warp_min(lo);
-    hi = warp_max(hi);
-    lo_in = warp_min(lo_in);
-    hi_in = warp_max(hi_in);
-    if ((threadIdx.x & 31) == 0) {
-        atomicMin(&st->cmin, lo);
-        atomicMax(&st->cmax, hi);
-        atomicMin(&st->cmin_in, lo_in);
-        atomicMax(&st->cmax_in, hi_in);
+    }
+}
+// Extremes of c = G / gm - E / em with numpy's FP32 operations (no contraction).
+template <bool VEC>
+__global__ void __launch_bounds__(256) combined_extremes(const uint16_t *__restrict__ g, const uint16_t *__restrict__ e,
+                                                         int64_t rows, uint32_t ny, int nx, int lanes,
+                                                         const int2 *__restrict__ inside, CombineStats *st) {
+    constexpr int V = VEC ? 8 : 1;
+    if (st->gmax == 0 || st->emax == 0) return;  // the host reports it
+    const Divisor by_g = divisor((float) st->gmax), by_e = divisor((float) st->emax);
+    const float inf = __int_as_float(0x7f800000);
+    float lo = inf, hi = -inf, lo_in = inf, hi_in = -inf;
+    int2 iv = make_int2(0, 0);
+    for_rows<VEC>(g, e, rows, nx, lanes, [&](int64_t r) { iv = __ldg(inside + (uint32_t) r % ny); },
+                  [&](int64_t, int x, const uint4 &wa, const uint4 &wb) {
+                      const uint32_t a[4] = {wa.x, wa.y, wa.z, wa.w}, b[4] = {wb.x, wb.y, wb.z, wb.w};
+                      float c[V + 1], l = inf, h = -inf;
+#pragma unroll
+                      for (int i = 0; i < V; i += 2) {
+                          const float2 p = combined(by_g, by_e, halves(a[i / 2]), halves(b[i / 2]));
+                          c[i] = p.x;
+                          c[i + 1] = p.y;  // (one voxel at a time: of no voxel)
+                      }
+#pragma unroll
+                      for (int i = 0; i < V; i++) {
+                          l = fminf(l, c[i]);
+                          h = fmaxf(h, c[i]);
+                      }
+                      lo = fminf(lo, l);
+                      hi = fmaxf(hi, h);
+                      if (x >= iv.x && x + V <= iv.y) {
+                          lo_in = fminf(lo_in, l);
+                          hi_in = fmaxf(hi_in, h);
+                      } else if (x + V > iv.x && x < iv.y) {
+#pragma unroll
+                          for (int i = 0; i < V; i++)
+                              if (x + i >= iv.x && x + i < iv.y) {
+                                  lo_in = fminf(lo_in, c[i]);
+                                  hi_in = fmaxf(hi_in, c[i]);
+                              }
+                      }
+                  });
+    const unsigned int k[4] = {lo <= hi ? ~fkey(lo) : 0u, lo <= hi ? fkey(hi) : 0u, lo_in <= hi_in ? ~fkey(lo_in) : 0u,
+                               lo_in <= hi_in ? fkey(hi_in) : 0u};
+    unsigned int *to = &st->ncmin;
+#pragma unroll
+    for (int i = 0; i < 4; i++) {
+        const unsigned int m = __reduce_max_sync(0xffffffffu, k[i]);
+        if ((threadIdx.x & 31) == 0 && m) atomicMax(to + i, m);
     }
 }
 
-struct ConvertScalars {
-    float gm, em, shift, denom, vmin, range;
-};
-
-__global__ void combined_convert(const uint16_t *__restrict__ g, const uint16_t *__restrict__ e,
-                                 uint16_t *__restrict__ out, int64_t rows, int64_t ny, int64_t nx, bool vec,
-                                 const int2 *__restrict__ inside, ConvertScalars s) {
-    for_chunks(rows, ny, nx, vec, [&](int64_t row, int y, int64_t x, int cnt) {
-        const int2 iv = __ldg(inside + y);
-        float a[8], b[8];
-        load8(g + row * nx + x, cnt, a);
-        load8(e + row * nx + x, cnt, b);
-        uint16_t q[8];
-        for (int i = 0; i < cnt; i++) {
-            const float c1 = __fdiv_rn(__fadd_rn(combined(a[i], b[i], s.gm, s.em), s.shift), s.denom);
-            const float t = __fmul_rn(__fdiv_rn(__fsub_rn(c1, s.vmin), s.range), 65535.0f);
-            const bool in = x + i >= iv.x && x + i < iv.y;
-            q[i] = (in && s.range > 0.0f) ? (uint16_t) __float2uint_rz(t) : (uint16_t) 0;
-        }
-        if (cnt == 8) {
-            uint4 w;
-            w.x = q[0] | ((uint32_t) q[1] << 16);
-            w.y = q[2] | ((uint32_t) q[3] << 16);
-            w.z = q[4] | ((uint32_t) q[5] << 16);
-            w.w = q[6] | ((uint32_t) q[7] << 16);
-            *reinterpret_cast<uint4 *>(out + row * nx + x) = w;
-        } else {
-            out[row * nx + x] = q[0];
-        }
-    });
+// any_inside / any_outside: whether the cylinder has voxels, and whether some are outside it.
+template <bool VEC>
+__global__ void __launch_bounds__(256) combined_convert(const uint16_t *__restrict__ g, const uint16_t *__restrict__ e,
+                                                        uint16_t *__restrict__ out, int64_t rows, uint32_t ny, int nx,
+                                                        int lanes, const int2 *__restrict__ inside, bool any_inside,
+                                                        bool any_outside, const CombineStats *__restrict__ st) {
+    constexpr int V = VEC ? 8 : 1;
+    if (st->gmax == 0 || st->emax == 0) return;
+    // The scalar steps in FP32, in numpy's order.
+    const Divisor by_g = divisor((float) st->gmax), by_e = divisor((float) st->emax);
+    const float shift = fabsf(key_float(~st->ncmin));
+    const Divisor by_denom = divisor(__fadd_rn(key_float(st->cmax), shift));
+    float vmin = 0.0f, vmax = 0.0f;
+    if (any_inside) {
+        const float lo = __fdiv_rn(__fadd_rn(key_float(~st->ncmin_in), shift), by_denom.b);
+        const float hi = __fdiv_rn(__fadd_rn(key_float(st->cmax_in), shift), by_denom.b);
+        // the host's std::min and std::max, which give the first argument for a NaN
+        vmin = any_outside ? (lo < 0.0f ? lo : 0.0f) : lo;
+        vmax = any_outside ? (0.0f < hi ? hi : 0.0f) : hi;
+    }
+    const Divisor by_range = divisor(__fsub_rn(vmax, vmin));
+    const bool some = by_range.b > 0.0f;
+    auto walk = [&](auto plain) {
+        constexpr bool PLAIN = decltype(plain)::value;
+        int2 iv = make_int2(0, 0);
+        for_rows<VEC>(
+            g, e, rows, nx, lanes, [&](int64_t r) { iv = __ldg(inside + (uint32_t) r % ny); },
+            [&](int64_t r, int x, const uint4 &wa, const uint4 &wb) {
+                const uint32_t a[4] = {wa.x, wa.y, wa.z, wa.w}, b[4] = {wb.x, wb.y, wb.z, wb.w};
+                uint32_t q[4] = {0u, 0u, 0u, 0u};
+                if (some && x + V > iv.x && x < iv.y) {
+#pragma unroll
+                    for (int i = 0; i < (V + 1) / 2; i++) {
+                        const float2 c = combined(by_g, by_e, halves(a[i]), halves(b[i]));
+                        const float2 c1 = by_denom.quotient<PLAIN>(__fadd2_rn(c, make_float2(shift, shift)));
+                        const float2 u = by_range.quotient<PLAIN>(__fadd2_rn(c1, make_float2(-vmin, -vmin)));
+                        float2 t = __fmul2_rn(u, make_float2(65535.0f, 65535.0f));
+                        // Inside the cylinder t lies in [0, 65535] (or is a NaN, taken as 0): the low bits of its
+                        // sum with 2^23 are its integer part.
+                        if (PLAIN) t = make_float2(fmaxf(t.x, 0.0f), fmaxf(t.y, 0.0f));
+                        t = __fadd2_rz(t, make_float2(8388608.0f, 8388608.0f));
+                        q[i] = __byte_perm(__float_as_uint(t.x), __float_as_uint(t.y), 0x5410);
+                    }
+                    if (x < iv.x || x + V > iv.y) {  // the cylinder's edge
+#pragma unroll
+                        for (int i = 0; i < V; i++)
+                            if (x + i < iv.x || x + i >= iv.y) q[i / 2] &= i % 2 ? 0x0000ffffu : 0xffff0000u;
+                    }
+                }
+                if constexpr (VEC) *reinterpret_cast<uint4 *>(out + r * nx + x) = make_uint4(q[0], q[1], q[2], q[3]);
+                else out[r * nx + x] = (uint16_t) q[0];
+            });
+    };
+    if (by_denom.plain || by_range.plain) walk(std::true_type{});
+    else walk(std::false_type{});
 }
 
 // numpy.linspace(-1, 1, n)[i] in FP64 (numpy: arange * step + start, last point = stop).
@@ -256,72 +357,43 @@ extern "C" int maxi_combine_fields(const uint16_t *gauss, const uint16_t *edt, i
     bool any_outside = false, any_inside = false;
     cylinder_intervals(ny, nx, inside, any_outside, any_inside);
 
+    std::unique_lock<std::mutex> hold;
     char *scratch = nullptr;
     const size_t iv_bytes = (size_t) ny * sizeof(int2);
-    const size_t bytes = 256 + round_up((int64_t) iv_bytes, 256);
-    if (cudaMallocAsync(reinterpret_cast<void **>(&scratch), bytes, st) != cudaSuccess) {
-        cudaGetLastError();
-        return set_error(MAXI_ERR_OUT_OF_MEMORY, "could not allocate %zu bytes of scratch", bytes);
-    }
+    if ((rc = acquire_scratch(256 + iv_bytes, hold, &scratch, "field combination"))) return rc;
     CombineStats *d_st = reinterpret_cast<CombineStats *>(scratch);
     int2 *d_iv = reinterpret_cast<int2 *>(scratch + 256);
-    CombineStats init{};
-    init.cmin = init.cmin_in = 0xffffffffu;
-    const bool vec = nx % 8 == 0 && ((reinterpret_cast<uintptr_t>(gauss) | reinterpret_cast<uintptr_t>(edt) |
-                                       reinterpret_cast<uintptr_t>(output)) & 15) == 0;
+    const bool aligned = ((reinterpret_cast<uintptr_t>(gauss) | reinterpret_cast<uintptr_t>(edt) |
+                           reinterpret_cast<uintptr_t>(output)) & 15) == 0;
+    const bool vec = nx % 8 == 0 && aligned;
     int dev = 0, sms = 148;
     cudaGetDevice(&dev);
     cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
-    const int64_t chunks = rows * (vec ? nx / 8 : nx);
-    const unsigned grid = (unsigned) std::min<int64_t>(ceil_div(chunks, 256), (int64_t) sms * 16);
     const int threads = 256;
+    int lanes = 1;
+    while (lanes < 32 && lanes * (vec ? 8 : 1) < nx) lanes *= 2;
+    const unsigned grid_flat = (unsigned) std::min<int64_t>(ceil_div(ceil_div(rows * nx, 8), threads), (int64_t) sms * 16);
+    const unsigned grid = (unsigned) std::min<int64_t>(ceil_div(rows * lanes, threads), (int64_t) sms * 16);
     CombineStats h{};
-    auto finish = [&](int code) {
-        cudaFreeAsync(scratch, st);
-        return code;
-    };
-    cudaError_t e;
-    if ((e = cudaMemcpyAsync(d_st, &init, sizeof(init), cudaMemcpyHostToDevice, st)) != cudaSuccess ||
-        (e = cudaMemcpyAsync(d_iv, inside.data(), iv_bytes, cudaMemcpyHostToDevice, st)) != cudaSuccess)
-        return finish(set_cuda_error(e, "combine_fields set-up"));
-    field_maxima<<<grid, threads, 0, st>>>(gauss, edt, rows, ny, nx, vec, d_st);
-    if ((e = cudaMemcpyAsync(&h, d_st, sizeof(h), cudaMemcpyDeviceToHost, st)) != cudaSuccess ||
-        (e = cudaStreamSynchronize(st)) != cudaSuccess)
-        return finish(set_cuda_error(e, "combine_fields maxima"));
-    if (h.gmax == 0 || h.emax == 0)
-        return finish(set_error(MAXI_ERR_INVALID_ARGUMENT,
-                                "the %s field is all zero (the combination divides by its maximum)",
-                                h.gmax == 0 ? "Gaussian" : "EDT"));
-    const float gm = (float) h.gmax, em = (float) h.emax;
-    combined_extremes<<<grid, threads, 0, st>>>(gauss, edt, rows, ny, nx, vec, d_iv, gm, em, d_st);
-    if ((e = cudaMemcpyAsync(&h, d_st, sizeof(h), cudaMemcpyDeviceToHost, st)) != cudaSuccess ||
-        (e = cudaStreamSynchronize(st)) != cudaSuccess)
-        return finish(set_cuda_error(e, "combine_fields extremes"));
-
-    // Scalar steps in FP32, in numpy's order (the x86-64 host rounds float
-    // arithmetic to single precision).
-    ConvertScalars s{};
-    s.gm = gm;
-    s.em = em;
-    volatile float cmin = key_float(h.cmin), cmax = key_float(h.cmax);
-    s.shift = std::fabs((float) cmin);
-    volatile float denom = cmax + s.shift;
-    s.denom = denom;
-    float vmin = 0.0f, vmax = 0.0f;
-    if (any_inside) {
-        volatile float lo = key_float(h.cmin_in) + s.shift, hi = key_float(h.cmax_in) + s.shift;
-        volatile float lo_d = lo / s.denom, hi_d = hi / s.denom;
-        vmin = any_outside ? std::min(0.0f, (float) lo_d) : (float) lo_d;
-        vmax = any_outside ? std::max(0.0f, (float) hi_d) : (float) hi_d;
+    cudaError_t e = cudaMemsetAsync(d_st, 0, sizeof(CombineStats), st);
+    if (e == cudaSuccess) e = cudaMemcpyAsync(d_iv, inside.data(), iv_bytes, cudaMemcpyHostToDevice, st);
+    if (e == cudaSuccess) {
+        field_maxima<<<grid_flat, threads, 0, st>>>(gauss, edt, rows * nx, aligned, d_st);
+        auto extremes = vec ? combined_extremes<true> : combined_extremes<false>;
+        extremes<<<grid, threads, 0, st>>>(gauss, edt, rows, (uint32_t) ny, (int) nx, lanes, d_iv, d_st);
+        auto convert = vec ? combined_convert<true> : combined_convert<false>;
+        convert<<<grid, threads, 0, st>>>(gauss, edt, output, rows, (uint32_t) ny, (int) nx, lanes, d_iv, any_inside,
+                                          any_outside, d_st);
+        e = cudaGetLastError();
     }
-    s.vmin = vmin;
-    volatile float range = vmax - vmin;
-    s.range = range;
-    combined_convert<<<grid, threads, 0, st>>>(gauss, edt, output, rows, ny, nx, vec, d_iv, s);
-    e = cudaGetLastError();
-    finish(0);
-    if (e == cudaSuccess) e = cudaStreamSynchronize(st);
-    return e == cudaSuccess ? MAXI_OK : set_cuda_error(e, "combine_fields convert");
+    if (e == cudaSuccess) e = cudaMemcpyAsync(&h, d_st, sizeof(h), cudaMemcpyDeviceToHost, st);
+    cudaError_t e2 = cudaStreamSynchronize(st);  // the scratch and the host intervals are free after it
+    if (e == cudaSuccess) e = e2;
+    if (e != cudaSuccess) return set_cuda_error(e, "combine_fields");
+    if (h.gmax == 0 || h.emax == 0)
+        return set_error(MAXI_ERR_INVALID_ARGUMENT, "the %s field is all zero (the combination divides by its maximum)",
+                         h.gmax == 0 ? "Gaussian" : "EDT");
+    return MAXI_OK;
 }
 
 extern "C" int maxi_mask_cylinder(uint16_t *field, int64_t nz, int64_t ny, int64_t nx, void *stream) {

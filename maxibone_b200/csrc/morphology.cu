@@ -37,12 +37,9 @@
 // busy, issue 57%), r = 20 7958 and 1611, r = 31 27900 and 3954; the uint8 form at r = 16
 // 3686 and 1156 (pack 101, unpack and combine 148).  Two words per thread instead of four
 // from radius 9 on: 1010 against 1074 us at r = 16 (twice the warps).
-#include <map>
-#include <mutex>
-#include <vector>
-
 #include "common.cuh"
 #include "host_util.h"
+#include "scratch.h"
 
 namespace maxi {
 namespace {
@@ -392,48 +389,6 @@ Partials partials(const MorphTile &t, const uint32_t *words) {
     return {words, t.nz, t.ny, t.pitch, t.radius, t.planes};
 }
 
-// Scratch kept between calls, one grow-only buffer per device: the pipeline applies
-// radius-16 spheres over and over, and mapping gigabytes afresh for each call would
-// cost more than the passes.  A call holds its device's buffer until it returns.
-struct Scratch {
-    std::mutex mu;
-    uint32_t *buf = nullptr;
-    size_t bytes = 0;
-};
-std::mutex g_scratch_mu;
-std::map<int, Scratch *> g_scratch;
-
-// Locks and returns the device's scratch, grown to `bytes`.
-int acquire_scratch(size_t bytes, std::unique_lock<std::mutex> &lock, uint32_t **p) {
-    int dev = 0;
-    cudaError_t e = cudaGetDevice(&dev);
-    if (e != cudaSuccess) return set_cuda_error(e, "cudaGetDevice");
-    Scratch *s;
-    {
-        std::lock_guard<std::mutex> lk(g_scratch_mu);
-        Scratch *&slot = g_scratch[dev];
-        if (!slot) slot = new Scratch();
-        s = slot;
-    }
-    lock = std::unique_lock<std::mutex>(s->mu);
-    if (s->bytes < bytes) {
-        if (s->buf) {
-            cudaDeviceSynchronize();  // earlier calls' work on the old buffer
-            cudaFree(s->buf);
-            s->buf = nullptr;
-            s->bytes = 0;
-        }
-        if (cudaMalloc(reinterpret_cast<void **>(&s->buf), bytes) != cudaSuccess) {
-            cudaGetLastError();
-            s->buf = nullptr;
-            return set_error(MAXI_ERR_OUT_OF_MEMORY, "could not allocate %zu bytes of morphology scratch", bytes);
-        }
-        s->bytes = bytes;
-    }
-    *p = s->buf;
-    return MAXI_OK;
-}
-
 template <bool DILATE>
 int morph_partial_planes(const uint32_t *in, uint32_t *partial, const MorphTile &t,
                          void (*kernel)(const uint32_t *, uint32_t *, const MorphTile), cudaStream_t st) {
@@ -457,7 +412,7 @@ int morph_run(const void *in, void *out, int64_t nz, int64_t ny, int64_t nx, int
     // (uint8: the packed input, then) the partial planes
     const int64_t packed_words = U8 ? round_up(words, 4) : 0;
     uint32_t *scratch = nullptr;
-    if ((rc = acquire_scratch((size_t) (packed_words + partial_words(t)) * sizeof(uint32_t), hold, &scratch))) return rc;
+    if ((rc = acquire_scratch((size_t) (packed_words + partial_words(t)) * sizeof(uint32_t), hold, &scratch, "morphology"))) return rc;
     uint32_t *partial = scratch + packed_words;
     const unsigned g = grid_for(words);
     if constexpr (U8) {
@@ -491,19 +446,6 @@ int check_shape(int64_t nz, int64_t ny, int64_t n_inner, int64_t radius) {
 }
 
 }  // namespace
-
-void release_morphology_scratch() {
-    std::lock_guard<std::mutex> lk(g_scratch_mu);
-    for (auto &kv : g_scratch) {
-        std::lock_guard<std::mutex> lk2(kv.second->mu);
-        if (kv.second->buf) {
-            cudaDeviceSynchronize();
-            cudaFree(kv.second->buf);
-            kv.second->buf = nullptr;
-            kv.second->bytes = 0;
-        }
-    }
-}
 
 }  // namespace maxi
 
