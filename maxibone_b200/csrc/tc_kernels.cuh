@@ -137,6 +137,70 @@ struct PassTaps {
     uint16_t lo[2 * kTcMaxRadiusWide + 1];
 };
 
+// The kernels' Toeplitz fill.  Row o of the matrix holds tap k - o - RA + R at
+// K element k, so the lanes of a warp read different taps; read from the
+// kernel parameters, that is one constant-cache access a lane and it took 70 us of a
+// 250 us launch at radius 128, 8-10 us of every launch at radius 16-32.
+// stage_taps copies the taps once into shared memory that the launch does not
+// use yet, zero-padded on both sides, and a second time one element on, so
+// that any two consecutive taps are one aligned 32-bit read; the copies lie 16
+// banks apart, which keeps the reads of even and odd rows off each other.
+// 256 x 512 x 768, radius 128: a z / y launch 247 -> 173 us, x 258 -> 221 us;
+// 200 x 344 x 456, radius 16: a repetition (z, y + x) 98 -> 78 us.
+constexpr int kTapPad = 136;    // zeros before tap 0: o up to 127, RA - R up to 7
+constexpr int kTapSpan = 640;   // K element 383 of row 0 lies at 136 + 383
+constexpr int kTapWords = kTapSpan / 2 + 16;     // words of one copy, with the bank offset
+constexpr int kTapStageBytes = 2 * kTapWords * 4;  // both copies of one coefficient set
+
+template <int THREADS>
+__device__ __forceinline__ void stage_taps(uint8_t *stage, const uint16_t *taps, int radius) {
+    uint16_t *even = reinterpret_cast<uint16_t *>(stage), *odd = even + 2 * kTapWords;
+    for (int i = threadIdx.x; i < kTapSpan; i += THREADS) {
+        const int t = i - kTapPad;
+        const uint16_t v = t >= 0 && t <= 2 * radius ? taps[t] : (uint16_t) 0;
+        even[i] = v;
+        if (i > 0) odd[i - 1] = v;
+        else odd[kTapSpan - 1] = 0;
+    }
+}
+
+// The words of Toeplitz row o: word c holds K elements 2c and 2c + 1.
+__device__ __forceinline__ const uint32_t *staged_row(const uint8_t *stage, const PassTaps &tp, int o, int shift) {
+    const int i = kTapPad - o + shift;  // K element 0
+    return reinterpret_cast<const uint32_t *>(stage) + (i & 1) * kTapWords + (i >> 1);
+}
+
+// Tensor-memory Toeplitz (z / y passes, transposed x pass): the two warps of a
+// lane quadrant write T_hi and T_lo of its 32 rows, or with one coefficient
+// set alternate blocks of T_hi.
+__device__ __forceinline__ void toeplitz_to_tmem(uint32_t base, const uint8_t *stage, const PassTaps &tp, int quad,
+                                                 int half, int lane, int shift) {
+    const uint32_t *w = staged_row(stage + (tp.hi_only ? 0 : half * kTapStageBytes), tp, quad * 32 + lane, shift);
+    const uint32_t col = base + ((uint32_t) (quad * 32) << 16) + (tp.hi_only ? 0 : half * tp.kcols);
+    for (int ch = tp.hi_only ? half : 0; ch < tp.kcols / 32; ch += tp.hi_only ? 2 : 1) {
+        uint32_t r[32];
+#pragma unroll
+        for (int j = 0; j < 32; j++) r[j] = w[ch * 32 + j];
+        tmem_st32(col + ch * 32, r);
+    }
+    tmem_st_wait();
+}
+
+// Shared-memory Toeplitz rows [row0, row0 + 128) of `rows` (K-major, 128-byte
+// swizzle), 16 bytes (8 K elements) a store.
+template <int THREADS, typename Perm>
+__device__ __forceinline__ void toeplitz_to_smem(uint8_t *tt, const uint8_t *stage, const PassTaps &tp, int row0,
+                                                 int rows, Perm out_of_row) {
+    const int nch = tp.kpa / 8;
+    for (int e = threadIdx.x; e < kXTN * nch; e += THREADS) {
+        const int sub = e & 7, rest = e >> 3;       // 8 chunks = one 128-byte swizzle row
+        const int n = rest % kXTN, kb = rest / kXTN;
+        const uint32_t *w = staged_row(stage, tp, out_of_row(n), tp.radius - tp.ra) + (kb * 8 + sub) * 4;
+        *reinterpret_cast<uint4 *>(tt + sw128_kmajor_offset(row0 + n, kb * 64 + sub * 8, rows)) =
+            make_uint4(w[0], w[1], w[2], w[3]);
+    }
+}
+
 // One column of a z / y pass: n_at axis tiles of TN x-columns at (x0, oth).
 // in_rows: the load map is over (x, axis, other) -- the y pass, and the z pass
 // reading [y][z][x] rows -- instead of the z pass's (x, y, z).
@@ -386,6 +450,9 @@ tc_strided_kernel(const __grid_constant__ CUtensorMap tmap, const __grid_constan
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const int64_t total = p.sched.total();
 
+    // The ring holds the staged taps until its first copy.
+    stage_taps<kThreads>(ring, tp.hi, tp.radius);
+    if (!tp.hi_only) stage_taps<kThreads>(ring + kTapStageBytes, tp.lo, tp.radius);
     if (threadIdx.x == 0) {
         for (int s = 0; s < STAGES; s++) { mbar_init(&full[s], 1); mbar_init(&empty[s], 1); }
         for (int d = 0; d < 2; d++) { mbar_init(&tfull[d], 1); mbar_init(&tempty[d], kEpiWarps); }
@@ -404,27 +471,9 @@ tc_strided_kernel(const __grid_constant__ CUtensorMap tmap, const __grid_constan
     tc_fence_after();
     const uint32_t tmem = *tmem_slot;
     if (warp >= 2) {
-        // Toeplitz halves into tensor memory, zero outside the band: the two
-        // warps of a lane quadrant write T_hi and T_lo of its 32 rows.
-        const int quad = warp & 3, lo_half = (warp - 2) >> 2;
-        const int o = quad * 32 + lane;
-        const uint16_t *taps = lo_half ? tp.lo : tp.hi;
-        for (int ch = 0; ch < tp.kcols / 32; ch++) {
-            uint32_t r[32];
-#pragma unroll
-            for (int j = 0; j < 32; j++) {
-                uint32_t v = 0;
-#pragma unroll
-                for (int e = 0; e < 2; e++) {
-                    const int k = 2 * (ch * 32 + j) + e, t = k - o;
-                    if (t >= 0 && t <= 2 * tp.radius && k < tp.kp) v |= (uint32_t) taps[t] << (16 * e);
-                }
-                r[j] = v;
-            }
-            tmem_st32(tmem + ((uint32_t) (quad * 32) << 16) + 2 * TN + (lo_half ? tp.kcols : 0) + ch * 32, r);
-        }
-        tmem_st_wait();
+        toeplitz_to_tmem(tmem + 2 * TN, ring, tp, warp & 3, (warp - 2) >> 2, lane, 0);
     }
+    fence_proxy_async_smem();  // the ring's first copies land on the staged taps
     tc_fence_before();
     __syncthreads();
     tc_fence_after();
@@ -614,14 +663,13 @@ tc_contig_kernel(const __grid_constant__ CUtensorMap tmap, const __grid_constant
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const int64_t total = p.sched.total();
 
-    for (int e = threadIdx.x; e < 2 * kXTN * tp.kpa; e += kXThreads) {
-        const int n = e / tp.kpa, j = e - n * tp.kpa;
-        const int o = n & (kXTN - 1);
-        const int t = j - o - tp.ra + tp.radius;  // tap index 0..2R
-        uint16_t v = 0;
-        if (t >= 0 && t <= 2 * tp.radius && j < tp.kp) v = n < kXTN ? tp.hi[t] : tp.lo[t];
-        *reinterpret_cast<uint16_t *>(tt + sw128_kmajor_offset(n, j, 2 * kXTN)) = v;
-    }
+    // The ring holds the staged taps until its first copy.
+    stage_taps<kXThreads>(ring, tp.hi, tp.radius);
+    if (!tp.hi_only) stage_taps<kXThreads>(ring + kTapStageBytes, tp.lo, tp.radius);
+    __syncthreads();
+    const auto identity = [](int n) { return n; };
+    toeplitz_to_smem<kXThreads>(tt, ring, tp, 0, 2 * kXTN, identity);
+    if (!tp.hi_only) toeplitz_to_smem<kXThreads>(tt, ring + kTapStageBytes, tp, kXTN, 2 * kXTN, identity);
     if (threadIdx.x == 0) {
         for (int s = 0; s < kXStages; s++) { mbar_init(&full[s], 1); mbar_init(&empty[s], 1); }
         for (int d = 0; d < 2; d++) { mbar_init(&tfull[d], 1); mbar_init(&tempty[d], kXEpiWarps); }
@@ -836,6 +884,9 @@ tc_contig_t_kernel(const __grid_constant__ CUtensorMap tmap, const __grid_consta
     const int64_t total = p.sched.total();
     constexpr uint32_t kAcc = 2 * kXtRows;              // accumulator columns; the Toeplitz halves follow
 
+    // The ring holds the staged taps until its first copy.
+    stage_taps<kXtThreads>(ring, tp.hi, tp.radius);
+    if (!tp.hi_only) stage_taps<kXtThreads>(ring + kTapStageBytes, tp.lo, tp.radius);
     if (threadIdx.x == 0) {
         for (int s = 0; s < kXtStages; s++) { mbar_init(&full[s], 1); mbar_init(&empty[s], 1); }
         for (int d = 0; d < 2; d++) { mbar_init(&tfull[d], 1); mbar_init(&tempty[d], kXtEpiWarps); }
@@ -854,27 +905,10 @@ tc_contig_t_kernel(const __grid_constant__ CUtensorMap tmap, const __grid_consta
     tc_fence_after();
     const uint32_t tmem = *tmem_slot;
     if (warp >= 2) {
-        // Tt^T halves into tensor memory: lane o holds x output o, K element j
-        // the tap j - o - RA + R (zero outside the band).
-        const int quad = warp & 3, lo_half = (warp - 2) >> 2;
-        const int o = quad * 32 + lane;
-        const uint16_t *taps = lo_half ? tp.lo : tp.hi;
-        for (int ch = 0; ch < tp.kcols / 32; ch++) {
-            uint32_t r[32];
-#pragma unroll
-            for (int j = 0; j < 32; j++) {
-                uint32_t v = 0;
-#pragma unroll
-                for (int e = 0; e < 2; e++) {
-                    const int k = 2 * (ch * 32 + j) + e, t = k - o - tp.ra + tp.radius;
-                    if (t >= 0 && t <= 2 * tp.radius && k < tp.kp) v |= (uint32_t) taps[t] << (16 * e);
-                }
-                r[j] = v;
-            }
-            tmem_st32(tmem + ((uint32_t) (quad * 32) << 16) + kAcc + (lo_half ? tp.kcols : 0) + ch * 32, r);
-        }
-        tmem_st_wait();
+        // Tt^T: lane o holds x output o, K element j the tap j - o - RA + R.
+        toeplitz_to_tmem(tmem + kAcc, ring, tp, warp & 3, (warp - 2) >> 2, lane, tp.radius - tp.ra);
     }
+    fence_proxy_async_smem();  // the ring's first copies land on the staged taps
     tc_fence_before();
     __syncthreads();
     tc_fence_after();

@@ -231,13 +231,10 @@ tc_yx_kernel(const __grid_constant__ CUtensorMap tmap, const __grid_constant__ C
 
     // T[n, j] = tap[j - n - RA + R]: the y pass's A (row n = output o, K = j)
     // and the x pass's B (row n = x-output, K = j) alike.
-    for (int e = threadIdx.x; e < kXTN * tp.kpa; e += kYxThreads) {
-        const int n = e / tp.kpa, j = e - n * tp.kpa;
-        const int t = j - yx_out_perm(n) - tp.ra + tp.radius;  // tap index 0..2R
-        uint16_t v = 0;
-        if (t >= 0 && t <= 2 * tp.radius && j < kp) v = tp.hi[t];
-        *reinterpret_cast<uint16_t *>(tt + sw128_kmajor_offset(n, j, kXTN)) = v;
-    }
+    // The ring holds the staged taps until its first copy.
+    stage_taps<kYxThreads>(ring, tp.hi, tp.radius);
+    __syncthreads();
+    toeplitz_to_smem<kYxThreads>(tt, ring, tp, 0, kXTN, [](int n) { return yx_out_perm(n); });
     if (threadIdx.x == 0) {
         for (int s = 0; s < stages; s++) { mbar_init(&full[s], 1); mbar_init(&empty[s], 1); }
         mbar_init(yfull, 1);
