@@ -160,7 +160,7 @@ int maxi_diffusion_in_memory(const uint8_t *voxels, int64_t nz, int64_t ny, int6
  * calls instead (one grow-only allocation per device), so repeated calls do
  * not map gigabytes each time; maxi_keep_device_buffers(0) restores the
  * default and frees them, as does maxi_release_cached_memory() (which also
- * frees the device scratch that the sphere morphology and the field steps keep
+ * frees the device scratch that the sphere morphology, the field steps and the histograms keep
  * and the 16 MB of pinned host memory that copies of pageable arrays go through).  Volumes larger than the device go to
  * the out-of-core form, as the reference's pybind module does
  * (src/pybind/diffusion-pybind.cc:40-45).

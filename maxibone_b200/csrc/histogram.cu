@@ -21,10 +21,11 @@
 // bin and no table.  Where no line fits, thresholds T[b] (the smallest counted value whose
 // bin is >= b) settle the fixed-point bin by one comparison each way.
 //
-// Counting, field_histogram.  One thread takes 8 consecutive voxels of a row (one 16-byte load
-// when rows are 16-byte aligned), adds runs of equal keys once and issues one 64-bit
-// reduction per run into the histogram (L2-resident at the pipeline's 2048 x 4096); each
-// block walks one contiguous range of rows.
+// Counting, field_histogram.  Large volumes: sorted by parts of the histogram, which are then
+// counted in shared memory (below).  The others, and bins too many for that: one thread takes 8
+// consecutive voxels of a row (one 16-byte load when rows are 16-byte aligned), adds runs of
+// equal keys once and issues one 64-bit reduction per run into the histogram (L2-resident at
+// the pipeline's 2048 x 4096); each block walks one contiguous range of rows.
 //
 // Counting, axis_histograms.  L2 takes about 150 to 190 G reductions per second on random
 // cells, shared memory 2300 G (measured), and a voxel counts in four histograms.  So each
@@ -37,10 +38,12 @@
 // shared histogram per row, 1611 us.
 #include <cmath>
 #include <mutex>
+#include <type_traits>
 #include <vector>
 
 #include "common.cuh"
 #include "host_util.h"
+#include "scratch.h"
 
 namespace maxi {
 namespace {
@@ -66,6 +69,14 @@ __device__ __forceinline__ int bin_of(const BinMap &m, int v) {
         else if ((uint32_t) v >= __ldg(m.T + b + 1)) b++;
     }
     return d <= (uint32_t) m.span ? b : -1;
+}
+
+// The same for a value within the range; anything outside it.
+template <bool EXACT = false>
+__device__ __forceinline__ int bin_in_range(const BinMap &m, int v) {
+    if (!EXACT) return bin_of(m, v);
+    const uint32_t d = (uint32_t) (v - m.lo);
+    return (int) (((uint64_t) d * m.mul_lo + m.offset) >> 32) + (int) (d * m.mul_hi);
 }
 
 // Voxels are read once: loaded evict-first, so the L2-resident bins stay in L2.
@@ -123,6 +134,366 @@ __global__ void field_histogram_kernel(const uint16_t *__restrict__ voxels, cons
             }
             if (run_key >= 0) atomicAdd(bins + run_key, (unsigned long long) run);
         }
+    }
+}
+
+// ---- field_histogram through partitioned keys ----------------------------------------
+//
+// The reductions of field_histogram_kernel hit random 64-bit cells of a histogram far larger
+// than any shared memory, 95 to 148 G a second whatever the launch (L2's rate), while shared
+// memory adds 2300 G a second.  So the cells are split into partitions of `group` field bins
+// that fit one SM's shared memory, and the voxels' cells are sorted by partition on the way:
+// partition_keys takes tiles of 16384 voxels, ranks each tile's 16-bit keys (the cell within
+// its partition) by partition with counters in shared memory, lines them up there and writes
+// them out in one run; count_partitions reads them back, partition after partition.  That moves
+// the voxels once and 2 bytes a voxel each way (158 partitions of a tile: about 70 keys in a
+// row).  Bound by instruction issue (57%, 54 instructions a voxel) and the tile's barriers;
+// a branch around tiles of air made the others slower (1.90 -> 1.97 ms: it ends the overlap of
+// one vector's loads with another's counting).
+// 512 x 1024 x 1024 against half resolution, 2048 x 4096 bins: 2.85 -> 1.90 ms (partition_keys
+// 1.36, count_partitions 0.50).
+constexpr int kKeyThreads = 512;
+constexpr int kKeyVecs = 4;                                // 8-voxel vectors per thread and tile
+constexpr int kTileVecs = kKeyThreads * kKeyVecs;
+constexpr int kTileKeys = kTileVecs * kVec;                // 16384
+constexpr int kMaxParts = 256;
+constexpr int kPartCells = 53248;                          // 208 KB of 32-bit counters
+constexpr int kGroupTiles = 4096;                          // whose runs a block lines up at a time
+constexpr int kMaxGroup = 4096;                            // fb / group below is exact up to here
+
+// n / d by a multiplication: exact for n * d < 2^32.
+struct SmallDiv {
+    uint32_t d, magic, one;
+    __device__ __forceinline__ uint32_t operator()(uint32_t n) const { return __umulhi(n, magic) + n * one; }
+};
+
+struct PartitionArgs {
+    const uint16_t *voxels, *field;
+    int64_t ny, nx;                     // the field's rows
+    int nX, x_start;
+    uint32_t nY, y_start, first_row, rows;  // this batch's rows of the volume
+    SmallDiv per_row, group;            // vectors per row, field bins per partition
+    BinMap vm, fm;
+    const int32_t *zmap, *ymap, *xmap;  // xmap: padded to whole vectors
+    int voxel_bins, field_bins, parts, tiles;
+    int pitch;                          // of starts: the tiles of a full batch, a multiple of 4
+    uint16_t *keys;                     // [tiles][kTileKeys], each tile's keys by partition
+    uint16_t *starts;                   // [parts + 1][pitch]: where a partition starts in a tile
+    uint32_t *totals;                   // [parts]: keys of a partition, all tiles
+    unsigned long long *bins;
+};
+
+// VEC8: rows of whole aligned vectors.
+template <bool VEC8, bool EXACT>
+__global__ void __launch_bounds__(kKeyThreads, 2) partition_keys(const PartitionArgs a) {
+    __shared__ __align__(16) uint16_t sorted[kTileKeys];
+    __shared__ uint32_t counts[kMaxParts], place[kMaxParts], sums[kMaxParts / 32];
+    constexpr uint32_t none = ~0u;  // part << 16 | rank of a voxel that is not counted
+    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+    if (tid < kMaxParts) counts[tid] = 0;
+    // VEC8: the batch's vectors lie one after another.
+    const uint4 *first = reinterpret_cast<const uint4 *>(a.voxels + (int64_t) a.first_row * a.nX);
+    const uint32_t vecs = a.rows * a.per_row.d;
+    uint32_t total = 0;  // of partition tid, over this block's tiles
+    __syncthreads();
+    for (int tile = blockIdx.x; tile < a.tiles; tile += gridDim.x) {
+        // Every load of the tile's voxels first, then the field's rows and values.
+        uint32_t key[kKeyVecs][kVec / 2], rank[kKeyVecs][kVec];  // two keys a word; part << 16 | rank
+        uint4 w[kKeyVecs];
+        int zi[kKeyVecs], yi[kKeyVecs], X[kKeyVecs];
+        const uint32_t vec0 = (uint32_t) tile * kTileVecs;
+#pragma unroll
+        for (int k = 0; k < kKeyVecs; k++) {
+            const uint32_t vec = vec0 + tid + kKeyThreads * k;
+            w[k] = make_uint4(0, 0, 0, 0);  // zero voxels are not counted
+            if (VEC8 && vec < vecs) w[k] = __ldcs(first + vec);
+        }
+        const uint32_t row0 = vec0 / a.per_row.d, col0 = vec0 - row0 * a.per_row.d;
+        const uint32_t Z0 = (a.first_row + row0) / a.nY, Y0 = a.first_row + row0 - Z0 * a.nY;
+#pragma unroll
+        for (int k = 0; k < kKeyVecs; k++) {
+            const uint32_t o = col0 + tid + kKeyThreads * k, r = a.per_row(o);
+            X[k] = (int) (o - r * a.per_row.d) * kVec;
+            uint32_t Z = Z0, Y = Y0 + r;
+            if (Y >= a.nY) Z += Y / a.nY, Y %= a.nY;
+            const bool live = row0 + r < a.rows && Y >= a.y_start;
+            zi[k] = live ? __ldg(a.zmap + Z) : 0;
+            yi[k] = live ? __ldg(a.ymap + Y) : 0;
+            if (!VEC8 && live) {
+                const uint16_t *vrow = a.voxels + ((int64_t) a.first_row + row0 + r) * a.nX + X[k];
+                uint32_t u[kVec];
+#pragma unroll
+                for (int j = 0; j < kVec; j++) u[j] = X[k] + j < a.nX ? __ldcs(vrow + j) : 0;
+                w[k] = make_uint4(u[0] | u[1] << 16, u[2] | u[3] << 16, u[4] | u[5] << 16, u[6] | u[7] << 16);
+            }
+            if (!live || X[k] < a.x_start) {  // voxels before the offset: zero
+                uint32_t u[4] = {w[k].x, w[k].y, w[k].z, w[k].w};
+                const int skip = live ? a.x_start - X[k] : kVec;
+#pragma unroll
+                for (int j = 0; j < kVec; j++)
+                    if (j < skip) u[j / 2] &= j & 1 ? 0x0000ffffu : 0xffff0000u;
+                w[k] = make_uint4(u[0], u[1], u[2], u[3]);
+            }
+        }
+#pragma unroll
+        for (int k = 0; k < kKeyVecs; k++) {
+            const int4 m0 = __ldg(reinterpret_cast<const int4 *>(a.xmap + X[k])),
+                       m1 = __ldg(reinterpret_cast<const int4 *>(a.xmap + X[k]) + 1);
+            const int at[kVec] = {m0.x, m0.y, m0.z, m0.w, m1.x, m1.y, m1.z, m1.w};
+            const uint32_t u[4] = {w[k].x, w[k].y, w[k].z, w[k].w};
+            const uint16_t *frow = a.field + ((int64_t) zi[k] * a.ny + yi[k]) * a.nx;
+            // G voxels to a field value: two where every pair of the warp's voxels reads one
+            // (a field at half resolution or less), whose bin and addition they then share.
+            auto rank_vector = [&](auto voxels_per_value) {
+                constexpr int G = decltype(voxels_per_value)::value;
+                uint32_t part[kVec / G], base[kVec / G], below[kVec / G], differ = 0;
+                int f[kVec / G];
+#pragma unroll
+                for (int i = 0; i < kVec / G; i++) f[i] = (int) __ldg(frow + at[G * i]);
+#pragma unroll
+                for (int i = 0; i < kVec / G; i++) {
+                    const int fb = bin_of<EXACT>(a.fm, f[i]);
+                    part[i] = fb >= 0 ? a.group((uint32_t) fb) : (uint32_t) kMaxParts;
+                    base[i] = ((uint32_t) fb - part[i] * a.group.d) * (uint32_t) a.voxel_bins;
+                    below[i] = fb >= 0 ? (uint32_t) a.vm.span + 1 : 0;
+                    differ |= part[i] ^ part[0];
+                }
+                bool counted[kVec];
+#pragma unroll
+                for (int j = 0; j < kVec; j += 2) {
+                    uint32_t q[2];
+#pragma unroll
+                    for (int h = 0; h < 2; h++) {
+                        const int v = (int) (h ? u[j / 2] >> 16 : u[j / 2] & 0xffffu);
+                        q[h] = base[(j + h) / G] + (uint32_t) bin_in_range<EXACT>(a.vm, v);
+                        counted[j + h] = (uint32_t) (v - a.vm.lo) < below[(j + h) / G];
+                    }
+                    key[k][j / 2] = __byte_perm(q[0], q[1], 0x5410);
+                }
+                // A warp whose 256 voxels all belong to one partition (a plateau's, or a smooth
+                // field's) ranks its own voxels and adds once; additions of many lanes to one
+                // counter would be taken one at a time.
+                const uint32_t p0 = __shfl_sync(0xffffffffu, part[0], 0);
+                if (__all_sync(0xffffffffu, (differ | (part[0] ^ p0)) == 0)) {
+                    uint32_t n = 0, m[kVec];
+#pragma unroll
+                    for (int j = 0; j < kVec; j++) {
+                        m[j] = __ballot_sync(0xffffffffu, counted[j]);
+                        n += __popc(m[j]);
+                    }
+                    uint32_t from = 0;
+                    if (lane == 0 && n) from = atomicAdd(&counts[p0], n);
+                    from = (p0 << 16) + __shfl_sync(0xffffffffu, from, 0);
+#pragma unroll
+                    for (int j = 0; j < kVec; j++) {
+                        rank[k][j] = counted[j] ? from + __popc(m[j] & ((1u << lane) - 1)) : none;
+                        from += __popc(m[j]);
+                    }
+                } else {
+#pragma unroll
+                    for (int i = 0; i < kVec / G; i++) {
+                        uint32_t n = 0;
+#pragma unroll
+                        for (int h = 0; h < G; h++) n += counted[G * i + h];
+                        uint32_t r = part[i] << 16;
+                        if (n) r += atomicAdd(&counts[part[i]], n);
+#pragma unroll
+                        for (int h = 0; h < G; h++) {
+                            rank[k][G * i + h] = counted[G * i + h] ? r : none;
+                            r += counted[G * i + h];
+                        }
+                    }
+                }
+            };
+            if (__all_sync(0xffffffffu, at[0] == at[1] && at[2] == at[3] && at[4] == at[5] && at[6] == at[7]))
+                rank_vector(std::integral_constant<int, 2>{});
+            else
+                rank_vector(std::integral_constant<int, 1>{});
+        }
+        __syncthreads();
+        // Partition starts: exclusive sums over the counts.
+        uint32_t count = 0, sum = 0;
+        if (warp < kMaxParts / 32) {
+            count = counts[tid];
+            counts[tid] = 0;
+            sum = count;
+#pragma unroll
+            for (int d = 1; d < 32; d *= 2) {
+                const uint32_t y = __shfl_up_sync(0xffffffffu, sum, d);
+                if (lane >= d) sum += y;
+            }
+            if (lane == 31) sums[warp] = sum;
+            total += count;
+        }
+        __syncthreads();
+        uint32_t all = 0, before = 0;
+#pragma unroll
+        for (int i = 0; i < kMaxParts / 32; i++) {
+            if (i < warp) before += sums[i];
+            all += sums[i];
+        }
+        if (tid < a.parts) {
+            place[tid] = before + sum - count;
+            a.starts[(int64_t) tid * a.pitch + tile] = (uint16_t) (before + sum - count);
+        }
+        if (tid == 0) a.starts[(int64_t) a.parts * a.pitch + tile] = (uint16_t) all;
+        __syncthreads();
+#pragma unroll
+        for (int k = 0; k < kKeyVecs; k++)
+#pragma unroll
+            for (int j = 0; j < kVec; j++)
+                if (rank[k][j] != none)
+                    sorted[place[rank[k][j] >> 16] + (rank[k][j] & 0xffffu)] =
+                        (uint16_t) (j & 1 ? key[k][j / 2] >> 16 : key[k][j / 2]);
+        __syncthreads();
+        // (The next tile's counts and sums change what this tile read before the barrier above;
+        // its keys go out before the next tile's scatter, two barriers on.)
+        uint4 *out = reinterpret_cast<uint4 *>(a.keys + (int64_t) tile * kTileKeys);
+        for (uint32_t i = tid; i * 8 < all; i += kKeyThreads) out[i] = reinterpret_cast<const uint4 *>(sorted)[i];
+    }
+    if (tid < a.parts && total) atomicAdd(a.totals + tid, total);
+}
+
+// Inclusive sum over the block's 1024 threads.
+__device__ __forceinline__ uint32_t block_sum(uint32_t v, uint32_t *sums) {
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+#pragma unroll
+    for (int d = 1; d < 32; d *= 2) {
+        const uint32_t y = __shfl_up_sync(0xffffffffu, v, d);
+        if (lane >= d) v += y;
+    }
+    __syncthreads();
+    if (lane == 31) sums[warp] = v;
+    __syncthreads();
+    uint32_t s = sums[lane];
+#pragma unroll
+    for (int d = 1; d < 32; d *= 2) {
+        const uint32_t y = __shfl_up_sync(0xffffffffu, s, d);
+        if (lane >= d) s += y;
+    }
+    const uint32_t before = __shfl_sync(0xffffffffu, s, (warp + 31) & 31);
+    return warp ? v + before : v;
+}
+
+// Counts the keys.  The (partition, tile) runs in order are split into one range of about equal
+// cost per block, cut between tiles, so that a partition that holds most keys (a field's
+// plateau) is shared by many blocks, and each block adds its counters to the bins once per
+// partition it meets.  Costs in keys: a run's look-up and partly filled loads, and a partition's
+// counters.
+constexpr uint32_t kRunCost = 16, kPartCost = 8192;
+
+__global__ void __launch_bounds__(1024) count_partitions(const PartitionArgs a) {
+    extern __shared__ uint32_t counters[];
+    __shared__ uint32_t upto[kMaxParts + 1], sums[32], cut[2];
+    __shared__ __align__(16) uint32_t chunks[kGroupTiles];
+    const int tid = threadIdx.x, lane = tid & 31;
+    for (int i = tid; i < kPartCells; i += 1024) counters[i] = 0;
+    {
+        const uint32_t keys = tid < a.parts ? __ldg(a.totals + tid) : 0;
+        const uint32_t s = block_sum(keys ? keys + kPartCost + kRunCost * a.tiles : 0, sums);
+        if (tid < a.parts) upto[tid + 1] = s;
+        if (tid == 0) upto[0] = 0;
+    }
+    __syncthreads();
+    const uint32_t n = upto[a.parts];
+    // The first run with a cost of `target` or more before it: partition part, tile cut[which]
+    // (up to `tiles`: the partition's end).
+    const int per = (a.tiles + 1023) / 1024;
+    auto find = [&](uint32_t target, int which, int &part) {
+        part = 0;
+        if (target > 0) part = __syncthreads_count(tid < a.parts && upto[tid + 1] < target);
+        const uint32_t into = target - upto[part], rest = into > kPartCost ? into - kPartCost : 0;
+        const uint16_t *lo = a.starts + (int64_t) part * a.pitch, *hi = lo + a.pitch;
+        const int t0 = min(a.tiles, tid * per), t1 = min(a.tiles, t0 + per);
+        auto cost = [&](int t) { return (uint32_t) __ldg(hi + t) - __ldg(lo + t) + kRunCost; };
+        uint32_t mine = 0;
+        for (int t = t0; t < t1; t++) mine += cost(t);
+        const uint32_t s = block_sum(mine, sums);
+        if (rest == 0) {
+            if (tid == 0) cut[which] = 0;
+        } else if (s >= rest && s - mine < rest) {
+            uint32_t c = s - mine;
+            int t = t0;
+            while (c < rest) c += cost(t++);
+            cut[which] = t;
+        }
+        __syncthreads();
+    };
+    if (n == 0) return;
+    int p0, p1;
+    find((uint32_t) ((uint64_t) n * blockIdx.x / gridDim.x), 0, p0);
+    find((uint32_t) ((uint64_t) n * (blockIdx.x + 1) / gridDim.x), 1, p1);
+    for (int p = p0; p <= p1; p++) {
+        const int tb = p == p0 ? (int) cut[0] : 0, te = p == p1 ? (int) cut[1] : a.tiles;
+        if (tb >= te || upto[p] == upto[p + 1]) continue;  // the same for every thread
+        const uint16_t *starts = a.starts + (int64_t) p * a.pitch;
+        for (int t0 = tb & ~3; t0 < te; t0 += kGroupTiles) {
+            // The next 4096 tiles' runs in chunks of 32 keys (a load of 8 lanes); a warp takes 32
+            // chunks in order at a time.
+            const int t = t0 + 4 * tid;
+            uint32_t mine[4], sum = 0;
+            const bool any = t < te;
+            const ushort4 l4 = any ? __ldg(reinterpret_cast<const ushort4 *>(starts + t)) : ushort4{},
+                          h4 = any ? __ldg(reinterpret_cast<const ushort4 *>(starts + a.pitch + t)) : ushort4{};
+            const uint32_t lo[4] = {l4.x, l4.y, l4.z, l4.w}, hi[4] = {h4.x, h4.y, h4.z, h4.w};
+#pragma unroll
+            for (int i = 0; i < 4; i++) {
+                mine[i] = t + i >= tb && t + i < te && hi[i] > lo[i] ? (hi[i] - (lo[i] & ~3u) + 31) / 32 : 0;
+                sum += mine[i];
+            }
+            uint32_t upper = block_sum(sum, sums) - sum;
+            uint4 c4;
+            c4.x = upper += mine[0];
+            c4.y = upper += mine[1];
+            c4.z = upper += mine[2];
+            c4.w = upper += mine[3];
+            reinterpret_cast<uint4 *>(chunks)[tid] = c4;
+            __syncthreads();
+            const uint32_t all = chunks[kGroupTiles - 1];
+            for (uint32_t c0 = (uint32_t) tid & ~31u; c0 < all; c0 += 1024) {
+                // Lane q looks up chunk c0 + q: the first tile whose sum is above it.
+                const uint32_t c = c0 + lane;
+                int at = 0;
+#pragma unroll
+                for (int d = kGroupTiles / 2; d > 0; d /= 2)
+                    if (chunks[at + d - 1] <= c) at += d;
+                uint32_t e = 0, base = 0;
+                if (c < all) {
+                    e = (uint32_t) __ldg(starts + t0 + at) | (uint32_t) __ldg(starts + a.pitch + t0 + at) << 16;
+                    base = ((e & 0xffffu) & ~3u) + (c - (at ? chunks[at - 1] : 0)) * 32;
+                }
+                uint2 w[8];
+                uint32_t i[8], run[8];
+#pragma unroll
+                for (int q = 0; q < 8; q++) {
+                    const int src = 4 * q + lane / 8;
+                    const int tq = t0 + __shfl_sync(0xffffffffu, at, src);
+                    run[q] = __shfl_sync(0xffffffffu, e, src);
+                    i[q] = __shfl_sync(0xffffffffu, base, src) + 4 * (lane & 7);
+                    if (i[q] < run[q] >> 16)
+                        w[q] = __ldcs(reinterpret_cast<const uint2 *>(a.keys + (int64_t) tq * kTileKeys + i[q]));
+                }
+#pragma unroll
+                for (int q = 0; q < 8; q++) {
+                    const uint32_t from = run[q] & 0xffffu, to = run[q] >> 16;
+                    if (i[q] >= from && i[q] < to) atomicAdd(counters + (w[q].x & 0xffffu), 1u);
+                    if (i[q] + 1 >= from && i[q] + 1 < to) atomicAdd(counters + (w[q].x >> 16), 1u);
+                    if (i[q] + 2 >= from && i[q] + 2 < to) atomicAdd(counters + (w[q].y & 0xffffu), 1u);
+                    if (i[q] + 3 >= from && i[q] + 3 < to) atomicAdd(counters + (w[q].y >> 16), 1u);
+                }
+            }
+            __syncthreads();
+        }
+        __syncthreads();
+        const int64_t first = (int64_t) p * a.group.d;
+        const int cells = (int) min((int64_t) a.group.d, a.field_bins - first) * a.voxel_bins;
+        unsigned long long *bins = a.bins + first * a.voxel_bins;
+        for (int i = tid; i < cells; i += 1024)
+            if (const uint32_t c = counters[i]) {
+                atomicAdd(bins + i, (unsigned long long) c);
+                counters[i] = 0;
+            }
+        __syncthreads();
     }
 }
 
@@ -565,6 +936,77 @@ int axis_launches(const uint16_t *voxels, int64_t nzl, int64_t Ny, int Nx, int64
                   width, per, rb, voxel_bins, (int) n_r);
 }
 
+// Voxels from which the partitioned form is the faster one, with at most kFewParts partitions
+// and with more.  Direct against partitioned, with torch's call, us: 3 partitions (256 x 512
+// bins) 59 / 53 at 2^20 voxels, 86 / 71 at 2^22, 154 / 88 at 2^23; 158 partitions (2048 x 4096)
+// 63 / 58 at 2^21, 63 / 78 at 2^22, 145 / 87 at 2^23.
+constexpr int kFewParts = 8;
+constexpr int64_t kFieldMinVoxelsFew = int64_t(1) << 20, kFieldMinVoxels = int64_t(3) << 21;
+// Vectors of one batch: the keys of 2^25 vectors take 512 MB.
+constexpr int64_t kBatchVecs = int64_t(1) << 25;
+
+SmallDiv small_div(uint32_t d) {
+    if (d == 1) return SmallDiv{1, 0, 1};
+    return SmallDiv{d, (uint32_t) (((uint64_t(1) << 32) + d - 1) / d), 0};
+}
+
+// field_histogram_kernel's call, partitioned, in batches of whole rows.
+struct FieldPlan {
+    bool partitioned;
+    int group, parts;
+    int64_t per_row, batch_rows, tiles;  // vectors per row; rows and tiles of a (full) batch
+    size_t o_totals, o_starts, o_keys, bytes;
+};
+
+FieldPlan field_plan(int64_t nZ, int64_t nY, int64_t nX, int64_t field_bins, int64_t voxel_bins, size_t tables) {
+    FieldPlan f{};
+    f.bytes = tables;
+    f.group = (int) std::min<int64_t>(std::min<int64_t>(kPartCells / voxel_bins, kMaxGroup), field_bins);
+    if (f.group < 1 || ceil_div(field_bins, f.group) > kMaxParts || nX > (1 << 18) || nZ * nY >= (int64_t(1) << 31) ||
+        nZ * nY * nX < (ceil_div(field_bins, f.group) <= kFewParts ? kFieldMinVoxelsFew : kFieldMinVoxels))
+        return f;
+    f.partitioned = true;
+    f.parts = (int) ceil_div(field_bins, f.group);
+    f.per_row = ceil_div(nX, kVec);
+    f.batch_rows = std::min(nZ * nY, kBatchVecs / f.per_row);
+    f.tiles = ceil_div(f.batch_rows * f.per_row, kTileVecs);
+    auto place = [&](size_t n) {
+        const size_t at = f.bytes;
+        f.bytes += (n + 255) / 256 * 256;
+        return at;
+    };
+    f.o_totals = place((size_t) f.parts * sizeof(uint32_t));
+    f.o_starts = place((size_t) (f.parts + 1) * round_up(f.tiles, 4) * sizeof(uint16_t));
+    f.o_keys = place((size_t) f.tiles * kTileKeys * sizeof(uint16_t));
+    return f;
+}
+
+int field_launches(const FieldPlan &f, PartitionArgs a, uint8_t *scratch, int64_t rows, bool vec, cudaStream_t st) {
+    const bool exact = !a.vm.T && !a.fm.T;
+    auto sort = vec ? (exact ? partition_keys<true, true> : partition_keys<true, false>)
+                    : (exact ? partition_keys<false, true> : partition_keys<false, false>);
+    const int smem = kPartCells * (int) sizeof(uint32_t), sms = sm_count();
+    cudaError_t e = cudaFuncSetAttribute(count_partitions, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
+    a.totals = reinterpret_cast<uint32_t *>(scratch + f.o_totals);
+    a.starts = reinterpret_cast<uint16_t *>(scratch + f.o_starts);
+    a.keys = reinterpret_cast<uint16_t *>(scratch + f.o_keys);
+    a.parts = f.parts;
+    a.pitch = (int) round_up(f.tiles, 4);
+    a.group = small_div((uint32_t) f.group);
+    a.per_row = small_div((uint32_t) f.per_row);
+    for (int64_t row = 0; row < rows && e == cudaSuccess; row += f.batch_rows) {
+        a.first_row = (uint32_t) row;
+        a.rows = (uint32_t) std::min(f.batch_rows, rows - row);
+        a.tiles = (int) ceil_div(a.rows * f.per_row, kTileVecs);
+        e = cudaMemsetAsync(a.totals, 0, f.parts * sizeof(uint32_t), st);
+        if (e != cudaSuccess) break;
+        sort<<<(unsigned) std::min(a.tiles, 2 * sms), kKeyThreads, 0, st>>>(a);
+        count_partitions<<<(unsigned) sms, 1024, smem, st>>>(a);
+        e = cudaGetLastError();
+    }
+    return e == cudaSuccess ? (int) MAXI_OK : set_cuda_error(e, "field histogram");
+}
+
 }  // namespace
 }  // namespace maxi
 
@@ -608,19 +1050,53 @@ extern "C" int maxi_field_histogram(const uint16_t *voxels, int64_t nZ, int64_t 
         volatile double t = (double) X * dx;
         xmap[X] = (uint32_t) std::min<int64_t>(nx - 1, (int64_t) std::floor((double) t));
     }
+    xmap.resize(round_up(nX, kVec), 0);
     DeviceTables t;
     const size_t o_vT = t.add(vT.data(), vT.size()), o_fT = t.add(fT.data(), fT.size());
     const size_t o_z = t.add(zmap.data(), zmap.size()), o_y = t.add(ymap.data(), ymap.size());
     const size_t o_x = t.add(xmap.data(), xmap.size());
-    rc = upload(t, st);
-    if (rc == MAXI_OK) {
-        if (!vT.empty()) vm.T = t.dev + o_vT;
-        if (!fT.empty()) fm.T = t.dev + o_fT;
-        const int32_t *zm = reinterpret_cast<const int32_t *>(t.dev + o_z);
-        const int32_t *ym = reinterpret_cast<const int32_t *>(t.dev + o_y);
-        const int32_t *xm = reinterpret_cast<const int32_t *>(t.dev + o_x);
-        auto *b = reinterpret_cast<unsigned long long *>(bins);
-        const bool vec = nX % kVec == 0 && reinterpret_cast<uintptr_t>(voxels) % 16 == 0;
+    const size_t tables = (t.host.size() * sizeof(uint32_t) + 255) / 256 * 256;
+    FieldPlan f = field_plan(nZ, nY, nX, field_bins, voxel_bins, tables);
+    std::unique_lock<std::mutex> lock;  // holds the scratch until the launches are done
+    uint8_t *scratch = nullptr;
+    rc = acquire_scratch(f.bytes, lock, &scratch, "histogram");
+    if (rc == MAXI_ERR_OUT_OF_MEMORY && f.partitioned) {  // the direct form needs the tables alone
+        clear_error();
+        if (lock) lock.unlock();
+        f.partitioned = false;
+        rc = acquire_scratch(tables, lock, &scratch, "histogram");
+    }
+    if (rc) return rc;
+    cudaError_t e = cudaMemcpyAsync(scratch, t.host.data(), t.host.size() * sizeof(uint32_t), cudaMemcpyHostToDevice, st);
+    if (e != cudaSuccess) return set_cuda_error(e, "histogram tables");
+    const uint32_t *dev = reinterpret_cast<const uint32_t *>(scratch);
+    if (!vT.empty()) vm.T = dev + o_vT;
+    if (!fT.empty()) fm.T = dev + o_fT;
+    const int32_t *zm = reinterpret_cast<const int32_t *>(dev + o_z);
+    const int32_t *ym = reinterpret_cast<const int32_t *>(dev + o_y);
+    const int32_t *xm = reinterpret_cast<const int32_t *>(dev + o_x);
+    auto *b = reinterpret_cast<unsigned long long *>(bins);
+    const bool vec = nX % kVec == 0 && reinterpret_cast<uintptr_t>(voxels) % 16 == 0;
+    if (f.partitioned) {
+        PartitionArgs a{};
+        a.voxels = voxels;
+        a.field = field;
+        a.ny = ny;
+        a.nx = nx;
+        a.nX = (int) nX;
+        a.x_start = (int) x_start;
+        a.nY = (uint32_t) nY;
+        a.y_start = (uint32_t) y_start;
+        a.vm = vm;
+        a.fm = fm;
+        a.zmap = zm;
+        a.ymap = ym;
+        a.xmap = xm;
+        a.voxel_bins = (int) voxel_bins;
+        a.field_bins = (int) field_bins;
+        a.bins = b;
+        rc = field_launches(f, a, scratch, nZ * nY, vec, st);
+    } else {
         const unsigned grid = (unsigned) std::min<int64_t>(nZ * nY, (int64_t) sm_count() * 16);
         if (vec)
             field_histogram_kernel<true><<<grid, 128, 0, st>>>(voxels, field, nZ, nY, (int) nX, ny, nx, y_start,
@@ -629,6 +1105,7 @@ extern "C" int maxi_field_histogram(const uint16_t *voxels, int64_t nZ, int64_t 
             field_histogram_kernel<false><<<grid, 256, 0, st>>>(voxels, field, nZ, nY, (int) nX, ny, nx, y_start,
                                                                 (int) x_start, vm, fm, zm, ym, xm, b, voxel_bins);
     }
+    t.dev = nullptr;  // the scratch stays
     return finish(t, st, rc, "field histogram");
 }
 

@@ -1,5 +1,5 @@
 // Device scratch kept between calls: one grow-only buffer per device, for the synchronous
-// entry points around the diffusion (morphology, field combination).
+// entry points around the diffusion (morphology, field combination, field histograms).
 // They are called over and over with the same sizes, and mapping memory afresh costs
 // 0.3 to 0.5 ms for the smallest buffer and tens of milliseconds for gigabytes.  A call
 // holds its device's buffer, locked, until its work on the device is done.

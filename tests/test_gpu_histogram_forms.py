@@ -4,7 +4,7 @@ import numpy as np
 import pytest
 
 import oracle
-from maxibone_b200.histograms import axis_histograms
+from maxibone_b200.histograms import axis_histograms, field_histogram
 
 pytestmark = pytest.mark.gpu
 
@@ -38,3 +38,31 @@ def test_axis_forms_match_oracle(gshape, nzb, offset, center, voxel_bins, vrange
     axis_histograms(voxels, offset, *got, center, vrange, 0)
     for g, w, name in zip(got, want, ("x", "y", "z", "r")):
         np.testing.assert_array_equal(g, w + np.uint64(3), err_msg=name)
+
+
+# field_histogram above the size from which its keys are partitioned: the pipeline's bins (158
+# partitions, the last with fewer field bins); odd rows and offsets; one partition; the most
+# partitions (one field bin each) and one more, which the direct form counts; ranges that need
+# thresholds; rows of one voxel, more of them than one batch holds; all voxels in one cell, which
+# many blocks then share; nothing to count.
+@pytest.mark.parametrize("vshape,fshape,offset,bins_shape,vrange,frange,constant", [
+    ((49, 360, 360), (25, 180, 180), (0, 0, 0), (2048, 4096), (1, 32000), (1, 65535), None),
+    ((65, 257, 257), (65, 257, 257), (0, 5, 13), (37, 1000), (1, 40000), (1, 65535), None),
+    ((2, 2100, 1000), (1, 700, 333), (0, 0, 8), (1, 1), (100, 60000), (1, 65535), None),
+    ((7, 1030, 900), (7, 103, 90), (1, 1029, 1), (256, 53248), (1, 65535), (1, 65535), None),
+    ((7, 1030, 900), (7, 103, 90), (0, 0, 0), (257, 53248), (1, 65535), (1, 65535), None),
+    ((11, 640, 640), (6, 320, 320), (0, 3, 2), (2304, 76), (1, 76), (1, 2304), None),
+    ((34, 1000003, 1), (9, 500002, 1), (0, 2, 0), (300, 512), (1, 32000), (1, 65535), None),
+    ((56, 333, 344), (28, 167, 172), (0, 0, 0), (2048, 4096), (1, 32000), (1, 65535), 31000),
+    ((56, 333, 344), (28, 167, 172), (0, 0, 0), (2048, 4096), (1, 32000), (1, 65535), 0),
+])
+def test_partitioned_field_histogram_matches_oracle(vshape, fshape, offset, bins_shape, vrange, frange, constant):
+    if constant is None:
+        voxels = _voxels(vshape, sum(vshape), 100 if vrange[1] < 100 else 45000)
+        field = _voxels(fshape, sum(fshape), 3000 if frange[1] < 3000 else 65536)
+    else:
+        voxels, field = np.full(vshape, constant, np.uint16), np.full(fshape, 65535, np.uint16)
+    want = oracle.field_histogram(voxels, field, offset, bins_shape, vrange, frange)
+    got = np.full(bins_shape, 3, np.uint64)
+    field_histogram(voxels, field, offset, got, vrange, frange, 0)
+    np.testing.assert_array_equal(got, want + np.uint64(3))
