@@ -18,6 +18,8 @@
 namespace maxi {
 namespace tc {
 
+constexpr int kBatchTN = strided_tn(kTcMaxRadius, false);  // the batches' z / y passes
+
 TcGeometry tc_geometry(int radius) {
     TcGeometry g;
     g.radius = radius;
@@ -29,7 +31,7 @@ TcGeometry tc_geometry(int radius) {
     return g;
 }
 
-// Fills the tile counts and the ten tensor maps of one volume.
+// Fills the tile counts and the twelve tensor maps of one volume.
 int tc_fill_volume(TcVol &vol, void *buf0, void *buf1, const uint32_t *packed_mask, uint16_t *out_u16,
                    float *field_out, int64_t nz, int64_t ny, int64_t nx, bool is_bf16, const TcGeometry &g) {
     vol = TcVol{};
@@ -41,8 +43,8 @@ int tc_fill_volume(TcVol &vol, void *buf0, void *buf1, const uint32_t *packed_ma
     vol.nz = nz; vol.ny = ny; vol.nx = nx;
     vol.n_at_z = (int) ceil_div(nz, kTM);
     vol.n_at_y = (int) ceil_div(ny, kTM);
-    vol.n_xc_z = (int) ceil_div(nx, StridedShape<true>::kTN);
-    vol.n_xc_y = (int) ceil_div(nx, StridedShape<false>::kTN);
+    vol.n_xc_z = (int) ceil_div(nx, kBatchTN);
+    vol.n_xc_y = (int) ceil_div(nx, kBatchTN);
     vol.n_xt = (int) ceil_div(nx, kXTN);
     vol.cols_z = (int64_t) vol.n_xc_z * ny;
     vol.cols_y = (int64_t) vol.n_xc_y * nz;
@@ -58,19 +60,22 @@ int tc_fill_volume(TcVol &vol, void *buf0, void *buf1, const uint32_t *packed_ma
         void *base = vol.buf[b];
         const cuuint64_t d3[3] = {(cuuint64_t) nx, (cuuint64_t) ny, (cuuint64_t) nz};
         const cuuint64_t s3[2] = {(cuuint64_t) (nx * 2), (cuuint64_t) (nx * ny * 2)};
-        const cuuint32_t boxz[3] = {64u, 1u, (cuuint32_t) g.kp_strided};
-        const cuuint32_t boxy[3] = {64u, (cuuint32_t) g.kp_strided, 1u};
+        const cuuint32_t boxz[3] = {64u, 1u, (cuuint32_t) kStridedRows};
+        const cuuint32_t boxy[3] = {64u, (cuuint32_t) kStridedRows, 1u};
+        const cuuint32_t boxyxin[3] = {64u, (cuuint32_t) g.kp_strided, 1u};
         const cuuint64_t dx[3] = {(cuuint64_t) nx, (cuuint64_t) (nz * ny), 1};
         const cuuint64_t sx[2] = {(cuuint64_t) (nx * 2), (cuuint64_t) (nx * nz * ny * 2)};
         const cuuint32_t boxx[3] = {64u, (cuuint32_t) kTM, 1u};
         const cuuint32_t boxs[3] = {32u, 32u, 1u};
         const cuuint64_t dr[3] = {(cuuint64_t) nx, (cuuint64_t) nz, (cuuint64_t) ny};
         const cuuint64_t sr[2] = {(cuuint64_t) (nx * 2), (cuuint64_t) (nz * nx * 2)};
-        const cuuint32_t boxr[3] = {64u, (cuuint32_t) g.kp_strided, 1u};
+        const cuuint32_t boxr[3] = {64u, (cuuint32_t) kStridedRows, 1u};
         const cuuint32_t boxyx[3] = {32u, 1u, 32u};
         if (enc(&vol.map[0][b], dt, 3, base, d3, s3, boxz, estr, CU_TENSOR_MAP_INTERLEAVE_NONE,
                 CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) != CUDA_SUCCESS ||
             enc(&vol.map[1][b], dt, 3, base, d3, s3, boxy, estr, CU_TENSOR_MAP_INTERLEAVE_NONE,
+                CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) != CUDA_SUCCESS ||
+            enc(&vol.yxin[b], dt, 3, base, d3, s3, boxyxin, estr, CU_TENSOR_MAP_INTERLEAVE_NONE,
                 CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) != CUDA_SUCCESS ||
             enc(&vol.map[2][b], dt, 3, base, dx, sx, boxx, estr, CU_TENSOR_MAP_INTERLEAVE_NONE,
                 CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) != CUDA_SUCCESS ||
@@ -94,7 +99,6 @@ cudaError_t tc_batch_pass(const TcVol *d_vols, const int64_t *d_prefix, int64_t 
     cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
     const unsigned grid = (unsigned) std::min<int64_t>(total, sms);
     CUtensorMap unused{};  // the batch kernels read their maps from the volume table
-    cudaError_t e;
     if (pass == 3) {
         if (!hi_only || g.radius > kTcMaxRadius || g.kp_contig != g.kp_strided) return cudaErrorInvalidValue;
         YxLaunch<ManyVolumesYx> p{};
@@ -113,8 +117,7 @@ cudaError_t tc_batch_pass(const TcVol *d_vols, const int64_t *d_prefix, int64_t 
                                         : tc_yx_kernel<__nv_bfloat16, MAXI_MASK_BITPACKED, false, ManyVolumesYx>)
                           : (final_pass ? tc_yx_kernel<__half, MAXI_MASK_BITPACKED, true, ManyVolumesYx>
                                         : tc_yx_kernel<__half, MAXI_MASK_BITPACKED, false, ManyVolumesYx>);
-        if ((e = cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, smem)) != cudaSuccess) return e;
-        k<<<grid, kYxThreads, smem, st>>>(unused, unused, p);
+        return launch_pass(k, false, grid, kYxThreads, smem, st, unused, unused, p);
     } else if (pass == 2) {
         ContigLaunch<ManyVolumesContig> p{};
         fill_pass_taps(p.taps, kernel, g.radius, g.ra, g.kp_contig, is_bf16, error_feedback, hi_only);
@@ -127,8 +130,7 @@ cudaError_t tc_batch_pass(const TcVol *d_vols, const int64_t *d_prefix, int64_t 
         const int smem = contig_smem_bytes_tc(p.taps.kp, p.taps.kpa);
         auto *k = is_bf16 ? tc_contig_kernel<__nv_bfloat16, MAXI_MASK_BITPACKED, ManyVolumesContig>
                           : tc_contig_kernel<__half, MAXI_MASK_BITPACKED, ManyVolumesContig>;
-        if ((e = cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, smem)) != cudaSuccess) return e;
-        k<<<grid, kXThreads, smem, st>>>(unused, p);
+        return launch_pass(k, false, grid, kXThreads, smem, st, unused, p);
     } else {
         const bool axis_z = pass == 0;
         StridedLaunch<ManyVolumesStrided> p{};
@@ -139,17 +141,14 @@ cudaError_t tc_batch_pass(const TcVol *d_vols, const int64_t *d_prefix, int64_t 
         p.sched.axis_z = axis_z ? 1 : 0;
         p.sched.in_buf = in_buf;
         p.sched.z_in_rows = (axis_z && rows_yz) ? 1 : 0;
-        p.sched.tn = axis_z ? StridedShape<true>::kTN : StridedShape<false>::kTN;
-        const int smem = strided_smem_bytes(p.taps.kp, p.sched.tn,
-                                            axis_z ? StridedShape<true>::kStages : StridedShape<false>::kStages);
+        p.sched.tn = kBatchTN;
+        const int smem = strided_smem_bytes(p.taps.kp, kBatchTN);
         auto *k = axis_z ? (is_bf16 ? tc_strided_kernel<__nv_bfloat16, true, 128, ManyVolumesStrided>
                                     : tc_strided_kernel<__half, true, 128, ManyVolumesStrided>)
                          : (is_bf16 ? tc_strided_kernel<__nv_bfloat16, false, 128, ManyVolumesStrided>
                                     : tc_strided_kernel<__half, false, 128, ManyVolumesStrided>);
-        if ((e = cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, smem)) != cudaSuccess) return e;
-        k<<<grid, kThreads, smem, st>>>(unused, unused, p);
+        return launch_pass(k, false, grid, strided_threads(kBatchTN), smem, st, unused, unused, p);
     }
-    return cudaGetLastError();
 }
 
 int tc_batch_read_and_clear_error() {

@@ -12,12 +12,13 @@ namespace maxi {
 namespace tc {
 
 // Device-table entry of one volume: tensor maps of the pass inputs
-// ([pass z/y/x][buffer]), of the y pass's stores, of the z pass's input in
-// [y][z][x] row order and of the fused y + x kernel's stores in that order
-// ([buffer]), the two ping-pong field buffers, the bit-packed mask, the final
+// ([pass z/y/x][buffer]) and of the fused y + x kernel's, of the y pass's stores,
+// of the z pass's input in [y][z][x] row order and of the fused y + x kernel's
+// stores in that order ([buffer]), the two ping-pong field buffers, the bit-packed mask, the final
 // outputs and the tile counts.
 struct alignas(64) TcVol {
     CUtensorMap map[3][2];
+    CUtensorMap yxin[2];    // fused y + x input ([buffer]), box 64 x KP x 1
     CUtensorMap ystore[2];
     CUtensorMap zrows[2];   // z-pass input read as [y][z][x] rows ([buffer])
     CUtensorMap yxrows[2];  // fused y + x stores to [y][z][x] rows ([buffer]), box 32 x 1 x 32

@@ -78,27 +78,33 @@ constexpr int kTM = 128;      // outputs along the axis (z / y) or rows (x) per 
 constexpr int kXTN = 128;     // x outputs per x-pass tile
 constexpr int kXStages = 2;   // TMA ring depth of the x pass
 constexpr int kPrefetch = 3;  // tiles prefetched into L2 ahead of the ring
-// L2 prefetch depth of the z / y passes (0: none; their TMA ring alone keeps
-// enough loads in flight).  Measured per 1024^3 BF16 z pass: 0.80 ms with
-// none, 0.85 with 1 tile, 0.86 with 2, 0.88 with 3, 1.04 with 6.
-constexpr int kPrefetchStrided = 0;
-constexpr int kEpiWarps = 8;  // z / y passes: two warps per TMEM lane quadrant, each drains half the columns
-constexpr int kThreads = 64 + 32 * kEpiWarps;  // warp 0 TMA, warp 1 MMA, warps 2..9 epilogue
+// z / y passes: eight epilogue warps, two to a TMEM lane quadrant, each drains half of a tile's
+// columns.  (One 32-column chunk a warp, with twice the warps: no faster, 1651 against 1655 us
+// at 200 x 344 x 456, and 0.5% slower at 1024^3.)
+constexpr int kEpiChunks = 2;  // 32-column chunks of a 128-column tile per warp
+__host__ __device__ constexpr int strided_epi_warps(int tn) { return tn == 128 ? 16 / kEpiChunks : 8; }
+// Warp 0 TMA, warp 1 MMA, then the epilogue.
+__host__ __device__ constexpr int strided_threads(int tn) { return 64 + 32 * strided_epi_warps(tn); }
 // The x pass's epilogue (mask, re-illumination, error feedback, stores) is the
 // longest: four warps per lane quadrant, each drains 32 of the 128 columns.
 constexpr int kXEpiWarps = 16;
 constexpr int kXThreads = 64 + 32 * kXEpiWarps;  // warp 0 TMA, warp 1 MMA, warps 2..17 epilogue
 
-// z / y passes: 128-column tiles (64 for radius > 64) in a 3-deep ring.  The
-// z pass stages its stores so one instruction writes 8 rows (its output rows
-// lie on different planes); the y pass writes each warp's 32 x 32 chunks with
-// TMA bulk stores.  Batches (radius <= 32) always use 128-column tiles.
-template <bool AXIS_Z> struct StridedShape {
-    static constexpr int kTN = 128;
-    static constexpr int kStages = 3;
-};
-constexpr int kStridedStages = 3;
-__host__ __device__ constexpr int strided_tn(int radius) { return radius <= 64 ? 128 : 64; }
+// z / y passes: 128-column tiles; 64 where two coefficient sets of more than 129 taps leave no
+// tensor memory for more.  A column's rows come in blocks of 128 rows through a ring, each row
+// once: a tile reads two or three blocks and frees the first.  (A ring of whole tiles' K rows
+// loads 1.25 to 3 times as many: at radius 128, 256 x 512 x 768, a launch took 173 us, 95 now;
+// at radius 32, 1024^3, 765 us, 684 now.  Blocks of 64 rows: 805 and 128 us, bound by the threads
+// that issue the loads and MMAs.)  The z pass stages its stores so one instruction writes 8 rows
+// (its output rows lie on different planes); the y pass writes each warp's 32 x 32 chunks with
+// TMA bulk stores.  No L2 prefetch: the ring alone keeps enough loads in flight.
+constexpr int kStridedRows = 128;  // of a block
+constexpr int kStridedMaxStages = 6;
+// Blocks in the ring: two tiles' worth.  More of them cost the HBM-bound passes the order of
+// their loads (1024^3, two blocks a tile: 0.684 ms with 4 stages, 0.742 with 6).
+__host__ __device__ constexpr int strided_stages(int kp) { return kp <= 2 * kStridedRows ? 4 : 6; }
+constexpr int kStridedChunkBytes = kStridedRows * 128;  // 64 columns of a block
+__host__ __device__ constexpr int strided_tn(int radius, bool hi_only) { return radius <= 64 || hi_only ? 128 : 64; }
 
 // Tensor memory of the strided passes (512 columns): accumulators [0, 2 TN),
 // then the Toeplitz halves, kcols columns each (K / 2 rounded up to 32: 96 up
@@ -106,14 +112,14 @@ __host__ __device__ constexpr int strided_tn(int radius) { return radius <= 64 ?
 constexpr uint32_t kTmemColsStrided = 512;
 __host__ __device__ constexpr int toeplitz_cols(int kp) { return ((kp / 2) + 31) / 32 * 32; }
 
-// Per-epilogue-warp staging: two 32-row x 32-column 16-bit buffers, 64-byte
-// rows with their 16-byte chunks XOR-swizzled by row / 2 (the y pass's store
-// map uses the same 64-byte swizzle; the z pass reads the rows back itself).
-constexpr int kStageWarpBytes = 2 * 32 * 64;
+// Per-epilogue-warp staging: 32 rows x 32 columns of 16-bit, 64-byte rows with
+// their 16-byte chunks XOR-swizzled by row / 2 (the y pass's store map uses the
+// same 64-byte swizzle; the z pass reads the rows back itself).
+constexpr int kStageWarpBytes = 32 * 64;
 
-__host__ __device__ constexpr int strided_smem_bytes(int kp, int tn, int stages) {
-    return 1024 /*alignment slack*/ + stages * (tn / 64) * kp * 128 /*B ring*/ + 1024 /*barriers, TMEM slot*/ +
-           kEpiWarps * kStageWarpBytes;
+__host__ __device__ constexpr int strided_smem_bytes(int kp, int tn) {
+    return 1024 /*alignment slack*/ + strided_stages(kp) * (tn / 64) * kStridedChunkBytes + 1024 /*barriers, TMEM slot*/ +
+           strided_epi_warps(tn) * kStageWarpBytes;
 }
 
 // x-pass staging of one epilogue warp's 32 rows x 32 columns of 16-bit output
@@ -125,11 +131,10 @@ __host__ __device__ constexpr int contig_smem_bytes_tc(int kp, int kpa) {
            1024 /*barriers, TMEM slot*/ + kXEpiWarps * kXStageWarpBytes;
 }
 
-// Taps and K extents of one pass.  K rows longer than a TMA box (256) are
-// loaded as nbox boxes of box_rows rows.
+// Taps and K extents of one pass.
 struct PassTaps {
     int radius, ra, kp, kpa;  // radius, x-pass left pad, K (multiple of 16), K rounded to 64
-    int kcols, nbox, box_rows;
+    int kcols;
     int error_feedback;
     int hi_only;  // one coefficient set (hi, rounded to keep the kernel's sum and second moment), no lo MMAs
     float inv_scale;
@@ -170,14 +175,14 @@ __device__ __forceinline__ const uint32_t *staged_row(const uint8_t *stage, cons
     return reinterpret_cast<const uint32_t *>(stage) + (i & 1) * kTapWords + (i >> 1);
 }
 
-// Tensor-memory Toeplitz (z / y passes, transposed x pass): the two warps of a
-// lane quadrant write T_hi and T_lo of its 32 rows, or with one coefficient
-// set alternate blocks of T_hi.
+// Tensor-memory Toeplitz (z / y passes, transposed x pass): the `parts` (2 or 4)
+// warps of a lane quadrant share the 32-column blocks of T_hi and T_lo.
 __device__ __forceinline__ void toeplitz_to_tmem(uint32_t base, const uint8_t *stage, const PassTaps &tp, int quad,
-                                                 int half, int lane, int shift) {
-    const uint32_t *w = staged_row(stage + (tp.hi_only ? 0 : half * kTapStageBytes), tp, quad * 32 + lane, shift);
-    const uint32_t col = base + ((uint32_t) (quad * 32) << 16) + (tp.hi_only ? 0 : half * tp.kcols);
-    for (int ch = tp.hi_only ? half : 0; ch < tp.kcols / 32; ch += tp.hi_only ? 2 : 1) {
+                                                 int part, int parts, int lane, int shift) {
+    const int sets = tp.hi_only ? 1 : 2, set = part % sets;
+    const uint32_t *w = staged_row(stage + set * kTapStageBytes, tp, quad * 32 + lane, shift);
+    const uint32_t col = base + ((uint32_t) (quad * 32) << 16) + set * tp.kcols;
+    for (int ch = part / sets; ch < tp.kcols / 32; ch += parts / sets) {
         uint32_t r[32];
 #pragma unroll
         for (int j = 0; j < 32; j++) r[j] = w[ch * 32 + j];
@@ -205,7 +210,7 @@ __device__ __forceinline__ void toeplitz_to_smem(uint8_t *tt, const uint8_t *sta
 // in_rows: the load map is over (x, axis, other) -- the y pass, and the z pass
 // reading [y][z][x] rows -- instead of the z pass's (x, y, z).
 struct StridedCol {
-    const CUtensorMap *in;       // load map (box 64 x KP along the axis)
+    const CUtensorMap *in;       // load map (box 64 x kStridedRows along the axis)
     const CUtensorMap *out_map;  // y pass: store map (box 32 x 32, 64-byte swizzle)
     void *out;
     int64_t A, stride_a, stride_o, nx;
@@ -430,31 +435,70 @@ template <class Sched> struct ContigLaunch {
     int final_pass;
 };
 
+// The passes are launched with programmatic stream serialization: a pass's blocks come up, with
+// barriers, tensor memory and the Toeplitz matrix, on the SMs that the pass before has left, and
+// touch the field only after pass_wait(), when that pass is complete and its writes are visible.
+// Every block waits, so a pass that is complete has all earlier ones behind it.  Without the
+// launch attribute both instructions do nothing.  It pays for one volume of fewer than
+// kOverlapVoxels (20 repetitions of 200 x 344 x 456: 1714 -> 1653 us, four of 256 x 512 x 768
+// at radius 128: 1726 -> 1673); ten of 1024^3 take 21.58 ms without it and 21.80 with it, a batch
+// of 16 volumes 7.28 and 7.33 ms.
+__device__ __forceinline__ void pass_prepare() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
+__device__ __forceinline__ void pass_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
+
+constexpr int64_t kOverlapVoxels = int64_t(1) << 28;
+
+template <typename... Params, typename... Args>
+cudaError_t launch_pass(void (*kernel)(Params...), bool overlap, int64_t grid, int threads, int smem, cudaStream_t st,
+                        const Args &...args) {
+    cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
+    if (e != cudaSuccess) return e;
+    cudaLaunchAttribute attr{};
+    attr.id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    attr.val.programmaticStreamSerializationAllowed = 1;
+    cudaLaunchConfig_t cfg{};
+    cfg.gridDim = dim3((unsigned) grid);
+    cfg.blockDim = dim3((unsigned) threads);
+    cfg.dynamicSmemBytes = (size_t) smem;
+    cfg.stream = st;
+    cfg.attrs = &attr;
+    cfg.numAttrs = overlap ? 1 : 0;
+    return cudaLaunchKernelEx(&cfg, kernel, args...);
+}
+
 // ---- z / y passes ------------------------------------------------------------------
 
 template <typename S, bool AXIS_Z, int TN, class Sched>
-__global__ void __launch_bounds__(kThreads, 1)
+__global__ void __launch_bounds__(strided_threads(TN), 1)
 tc_strided_kernel(const __grid_constant__ CUtensorMap tmap, const __grid_constant__ CUtensorMap tmap_out,
                   const __grid_constant__ StridedLaunch<Sched> p) {
-    constexpr int STAGES = kStridedStages, CHUNKS = TN / 64;
+    constexpr int CHUNKS = TN / 64, kStageBytes = CHUNKS * kStridedChunkBytes;
+    constexpr int kEpiWarps = strided_epi_warps(TN);
     const PassTaps &tp = p.taps;
+    const int stages = strided_stages(tp.kp);
+    pass_prepare();
     extern __shared__ uint8_t smem_raw[];
     const uint32_t raw = smem_u32(smem_raw);
     uint8_t *ring = smem_raw + (((raw + 1023) & ~1023u) - raw);
-    const int stage_bytes = CHUNKS * tp.kp * 128;
-    uint64_t *bars = reinterpret_cast<uint64_t *>(ring + STAGES * stage_bytes);
-    uint64_t *full = bars, *empty = bars + STAGES, *tfull = bars + 2 * STAGES, *tempty = bars + 2 * STAGES + 2;
-    uint64_t *drain = bars + 2 * STAGES + 4;
-    uint32_t *tmem_slot = reinterpret_cast<uint32_t *>(bars + 2 * STAGES + 5);
+    constexpr int kStep = kTM / kStridedRows;                          // blocks from tile to tile
+    const int nb = (tp.kp + kStridedRows - 1) / kStridedRows;          // blocks per tile
+    // Blocks of a column: those whose rows lie all past the volume's end are zeros and left out.
+    auto blocks = [&](const StridedCol &c) {
+        return min((c.n_at - 1) * kStep + nb, (int) ((c.A + tp.radius + kStridedRows - 1) / kStridedRows));
+    };
+    uint64_t *bars = reinterpret_cast<uint64_t *>(ring + stages * kStageBytes);
+    uint64_t *full = bars, *empty = bars + kStridedMaxStages, *tfull = bars + 2 * kStridedMaxStages, *tempty = tfull + 2;
+    uint64_t *drain = tfull + 4;
+    uint32_t *tmem_slot = reinterpret_cast<uint32_t *>(tfull + 5);
     uint8_t *stage_out = reinterpret_cast<uint8_t *>(bars) + 1024;  // 1024-byte aligned
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const int64_t total = p.sched.total();
 
     // The ring holds the staged taps until its first copy.
-    stage_taps<kThreads>(ring, tp.hi, tp.radius);
-    if (!tp.hi_only) stage_taps<kThreads>(ring + kTapStageBytes, tp.lo, tp.radius);
+    stage_taps<strided_threads(TN)>(ring, tp.hi, tp.radius);
+    if (!tp.hi_only) stage_taps<strided_threads(TN)>(ring + kTapStageBytes, tp.lo, tp.radius);
     if (threadIdx.x == 0) {
-        for (int s = 0; s < STAGES; s++) { mbar_init(&full[s], 1); mbar_init(&empty[s], 1); }
+        for (int s = 0; s < stages; s++) { mbar_init(&full[s], 1); mbar_init(&empty[s], 1); }
         for (int d = 0; d < 2; d++) { mbar_init(&tfull[d], 1); mbar_init(&tempty[d], kEpiWarps); }
         mbar_init(drain, 1);
         fence_barrier_init();
@@ -471,87 +515,92 @@ tc_strided_kernel(const __grid_constant__ CUtensorMap tmap, const __grid_constan
     tc_fence_after();
     const uint32_t tmem = *tmem_slot;
     if (warp >= 2) {
-        toeplitz_to_tmem(tmem + 2 * TN, ring, tp, warp & 3, (warp - 2) >> 2, lane, 0);
+        toeplitz_to_tmem(tmem + 2 * TN, ring, tp, warp & 3, (warp - 2) >> 2, kEpiWarps / 4, lane, 0);
     }
     fence_proxy_async_smem();  // the ring's first copies land on the staged taps
     tc_fence_before();
     __syncthreads();
     tc_fence_after();
 
+    pass_wait();
+    // Block b of a column holds the kStridedRows rows from b * kStridedRows - radius on; tile at
+    // reads the nb blocks from at * kStep on, so that every row of a column is loaded once.
     if (warp == 0 && lane == 0) {
-        // TMA producer; L2 prefetch kPrefetch tiles ahead, into this CTA's next column.
-        int64_t tl = 0;
-        bool ok = true;
-        int64_t g = blockIdx.x;
+        // TMA producer.  Stages and phases advance by increments here and below: the passes over
+        // L2-resident volumes wait on these two threads (64-bit remainders by the ring's depth
+        // alone took 6% of them).
+        int s = 0;
+        uint32_t ph = 0;
+        bool ok = true, wrapped = false;
         typename Sched::Cursor cc;
-        StridedCol cur = p.sched.col(g < total ? g : 0, &tmap, &tmap_out, cc), nxt = cur;
-        for (; ok && g < total; g += gridDim.x) {
-            const bool has_next = g + gridDim.x < total;
-            if (has_next) nxt = p.sched.col(g + gridDim.x, &tmap, &tmap_out, cc);
-            for (int at = 0; at < cur.n_at; at++, tl++) {
-                const int s = (int) (tl % STAGES);
-                const uint32_t ph = (uint32_t) ((tl / STAGES) & 1);
+        for (int64_t g = blockIdx.x; ok && g < total; g += gridDim.x) {
+            const StridedCol cur = p.sched.col(g, &tmap, &tmap_out, cc);
+            const int n_blocks = blocks(cur);
+            for (int b = 0, a = -tp.radius; b < n_blocks; b++, a += kStridedRows) {
                 if (!mbar_wait(&empty[s], ph ^ 1, 1)) { ok = false; break; }
-                if (kPrefetchStrided > 0) {
-                    const int ap = at + kPrefetchStrided;
-                    const CUtensorMap *pm = nullptr;
-                    int px = 0, po = 0, pa = 0, pr = 0;
-                    if (ap < cur.n_at) { pm = cur.in; px = cur.x0; po = cur.oth; pa = ap; pr = cur.in_rows; }
-                    else if (has_next && ap - cur.n_at < nxt.n_at) {
-                        pm = nxt.in; px = nxt.x0; po = nxt.oth; pa = ap - cur.n_at; pr = nxt.in_rows;
-                    }
-                    if (pm) {
-                        for (int c = 0; c < CHUNKS; c++)
-                            for (int b = 0; b < tp.nbox; b++) {
-                                const int a = pa * kTM - tp.radius + b * tp.box_rows;
-                                if (pr) tma_prefetch_3d(pm, px + 64 * c, a, po);
-                                else tma_prefetch_3d(pm, px + 64 * c, po, a);
-                            }
-                    }
+                mbar_arrive_expect_tx(&full[s], kStageBytes);
+                uint8_t *dst = ring + s * kStageBytes;
+#pragma unroll
+                for (int c = 0; c < CHUNKS; c++) {
+                    if (cur.in_rows) tma_load_3d(dst + c * kStridedChunkBytes, cur.in, cur.x0 + 64 * c, a, cur.oth, &full[s]);
+                    else tma_load_3d(dst + c * kStridedChunkBytes, cur.in, cur.x0 + 64 * c, cur.oth, a, &full[s]);
                 }
-                const int a_in = at * kTM - tp.radius;
-                mbar_arrive_expect_tx(&full[s], stage_bytes);
-                for (int c = 0; c < CHUNKS; c++)
-                    for (int b = 0; b < tp.nbox; b++) {
-                        uint8_t *dst = ring + s * stage_bytes + c * tp.kp * 128 + b * tp.box_rows * 128;
-                        const int a = a_in + b * tp.box_rows;
-                        if (cur.in_rows) tma_load_3d(dst, cur.in, cur.x0 + 64 * c, a, cur.oth, &full[s]);
-                        else tma_load_3d(dst, cur.in, cur.x0 + 64 * c, cur.oth, a, &full[s]);
-                    }
+                if (++s == stages) s = 0, ph ^= 1, wrapped = true;
             }
-            cur = nxt;
         }
         // The copies this thread started land before the CTA can exit (the last
         // use of each ring stage; bounded, so an aborted run still ends).
-        for (int64_t k = tl - STAGES; k < tl; k++)
-            if (k >= 0) mbar_wait(&full[k % STAGES], (uint32_t) ((k / STAGES) & 1), 1);
+        for (int k = 0; k < stages; k++)
+            if (k < s || wrapped) mbar_wait(&full[k], k < s ? ph : ph ^ 1, 1);
     } else if (warp == 1 && lane == 0) {
         // MMA issuer.
         const uint32_t fmt = std::is_same<S, __nv_bfloat16>::value ? 1u : 0u;
         const uint32_t idesc = idesc_f16(fmt, 0 /*A K-major*/, 1 /*B MN-major*/, kTM, TN);
-        const uint32_t b0 = smem_u32(ring);
-        int64_t tl = 0;
+        const uint64_t bd0 = smem_desc_sw128(smem_u32(ring), kStridedChunkBytes, 1024);
+        const uint32_t a_hi = tmem + 2 * TN, a_lo = a_hi + tp.kcols;
+        const bool two = !tp.hi_only;
+        // Block q, the tile's first, lies in stage s; the next one to wait for, `ahead` on, in sl.
+        int s = 0, sl = 0, ahead = 0;
+        uint32_t phl = 0, tl = 0;
         bool ok = true;
         typename Sched::Cursor cc;
         for (int64_t g = blockIdx.x; ok && g < total; g += gridDim.x) {
-            const int n_at = p.sched.col(g, &tmap, &tmap_out, cc).n_at;
-            for (int at = 0; at < n_at; at++, tl++) {
-                const int s = (int) (tl % STAGES);
-                const uint32_t ph = (uint32_t) ((tl / STAGES) & 1);
-                const int d = (int) (tl & 1);
-                const uint32_t dph = (uint32_t) ((tl >> 1) & 1);
-                if (!mbar_wait(&full[s], ph, 1) || !mbar_wait(&tempty[d], dph ^ 1, 3)) { ok = false; break; }
+            const StridedCol c = p.sched.col(g, &tmap, &tmap_out, cc);
+            const int n_blocks = blocks(c);
+            for (int at = 0; at < c.n_at; at++, tl++) {
+                const int n_tile = min(nb, n_blocks - at * kStep);
+                const uint32_t d = tl & 1;
+                if (!mbar_wait(&tempty[d], ((tl >> 1) & 1) ^ 1, 3)) { ok = false; break; }
                 tc_fence_after();
                 const uint32_t dt = tmem + d * TN;
-                // K step ks: 16 rows of the field tile (2048 bytes on, i.e. +128 in the
-                // descriptor's address field) and 8 tensor-memory columns of T.
-                const uint64_t bd = smem_desc_sw128(b0 + s * stage_bytes, tp.kp * 128, 1024);
-                const uint32_t a_hi = tmem + 2 * TN, a_lo = a_hi + tp.kcols;
-                for (int ks = 0; ks < tp.kp / 16; ks++) {
-                    umma_f16_ts(dt, a_hi + ks * 8, bd + (uint64_t) (ks * 128), idesc, ks > 0 ? 1u : 0u);
-                    if (!tp.hi_only) umma_f16_ts(dt, a_lo + ks * 8, bd + (uint64_t) (ks * 128), idesc, 1u);
+                uint32_t a = 0, more = 0;
+                int left = tp.kp / 16;
+                for (int b = 0, st = s; b < n_tile; b++) {
+                    if (b >= ahead) {
+                        if (!(ok = mbar_wait(&full[sl], phl, 1))) break;
+                        if (++sl == stages) sl = 0, phl ^= 1;
+                        ahead++;
+                        tc_fence_after();
+                    }
+                    // K step by K step: 16 rows on (2048 bytes, i.e. +128 in the descriptor's
+                    // address field) and 8 tensor-memory columns of T.
+                    uint64_t bd = bd0 + (uint64_t) (st * (kStageBytes / 16));
+                    const int n = min(kStridedRows / 16, left);
+                    left -= n;
+                    for (int ks = 0; ks < n; ks++, bd += 128, a += 8, more = 1) {
+                        umma_f16_ts(dt, a_hi + a, bd, idesc, more);
+                        if (two) umma_f16_ts(dt, a_lo + a, bd, idesc, 1u);
+                    }
+                    if (++st == stages) st = 0;
                 }
-                umma_commit(&empty[s]);
+                if (!ok) break;
+                // Blocks that no later tile of the column reads.
+                const int done = at + 1 < c.n_at ? kStep : n_tile;
+                for (int b = 0; b < done; b++) {
+                    umma_commit(&empty[s]);
+                    if (++s == stages) s = 0;
+                }
+                ahead -= done;
                 umma_commit(&tfull[d]);
             }
         }
@@ -561,9 +610,9 @@ tc_strided_kernel(const __grid_constant__ CUtensorMap tmap, const __grid_constan
     } else if (warp >= 2) {
         // Epilogue: TMEM -> registers -> storage type -> global.
         const int quad = warp & 3;           // TMEM lane quadrant this warp may access
-        const int half = (warp - 2) >> 2;    // which half of the columns it drains
+        const int part = (warp - 2) >> 2;    // which columns it drains
+        constexpr int kChunks = TN / 32 / (kEpiWarps / 4);
         uint8_t *stg = stage_out + (warp - 2) * kStageWarpBytes;
-        int sbuf = 0;
         int64_t tl = 0;
         bool ok = true;
         typename Sched::Cursor cc;
@@ -575,62 +624,57 @@ tc_strided_kernel(const __grid_constant__ CUtensorMap tmap, const __grid_constan
                 const uint32_t dph = (uint32_t) ((tl >> 1) & 1);
                 if (!mbar_wait(&tfull[d], dph, 2)) { ok = false; break; }
                 tc_fence_after();
-                const int c0 = half * CHUNKS;  // this warp's 32-column chunks
-                const uint32_t tbase = tmem + ((uint32_t) (quad * 32) << 16) + d * TN;
+                const int a0 = at * kTM + quad * 32;  // the warp's first output
 #pragma unroll
-                for (int cc = 0; cc < CHUNKS; cc++) {
+                for (int ch = 0; ch < kChunks; ch++) {
+                    const int col = (part * kChunks + ch) * 32;
+                    const int64_t xb = (int64_t) c.x0 + col;
+                    const bool live = a0 < c.A && xb < c.nx;  // warp-uniform
                     float va[32];
-                    __syncwarp();
-                    tmem_ld32(tbase + (c0 + cc) * 32, va);
+                    if (live) {
+                        __syncwarp();
+                        tmem_ld32(tmem + ((uint32_t) (quad * 32) << 16) + d * TN + col, va);
+                    }
+                    if (ch == kChunks - 1) {  // the accumulator is free once read, before the rounding
+                        tc_fence_before();
+                        __syncwarp();
+                        if (lane == 0) mbar_arrive(&tempty[d]);
+                    }
+                    if (!live) continue;
                     uint32_t qd[16], q[16];  // q[i]: voxels 2i, 2i + 1
                     narrow32_pairs<S, false>(va, tp.inv_scale, tp.error_feedback, 0u, 0xffffffffu, qd);
                     pairs_to_adjacent(qd, q);
-                    const int64_t xb = (int64_t) c.x0 + (c0 + cc) * 32;
-                    if (AXIS_Z) {
-                        // z pass: lanes' rows lie on different planes (2 MB apart at 1024^2);
-                        // stage the 32 x 32 chunk and write 8 rows (8 x 64 bytes) per instruction.
-                        __syncwarp();
+                    if (!AXIS_Z && lane == 0) bulk_wait_read<0>();  // the last store has read the buffer
+                    __syncwarp();
 #pragma unroll
-                        for (int i = 0; i < 4; i++)
-                            *reinterpret_cast<uint4 *>(stg + lane * 64 + ((i ^ ((lane >> 1) & 3)) << 4)) =
-                                make_uint4(q[4 * i], q[4 * i + 1], q[4 * i + 2], q[4 * i + 3]);
+                    for (int i = 0; i < 4; i++)
+                        *reinterpret_cast<uint4 *>(stg + lane * 64 + ((i ^ ((lane >> 1) & 3)) << 4)) =
+                            make_uint4(q[4 * i], q[4 * i + 1], q[4 * i + 2], q[4 * i + 3]);
+                    if (AXIS_Z) {
+                        // z pass: the rows lie on different planes (2 MB apart at 1024^2); 8 rows
+                        // (8 x 64 bytes) per instruction.
                         __syncwarp();
                         const int sub = lane & 3, rsub = lane >> 2;
 #pragma unroll
                         for (int r4 = 0; r4 < 4; r4++) {
                             const int rr = r4 * 8 + rsub;
-                            const int64_t ar = (int64_t) at * kTM + quad * 32 + rr;
+                            const int64_t ar = a0 + rr;
                             const uint4 w = *reinterpret_cast<const uint4 *>(stg + rr * 64 + ((sub ^ ((rr >> 1) & 3)) << 4));
                             if (ar < c.A && xb + sub * 8 < c.nx)
                                 *reinterpret_cast<uint4 *>(out + ar * c.stride_a + (int64_t) c.oth * c.stride_o + xb +
                                                            sub * 8) = w;
                         }
                     } else {
-                        // y pass: TMA store of the warp's 32 rows x 32 columns (64-byte swizzle of
-                        // the store map; the map clips rows and columns outside the volume).
-                        if (lane == 0) bulk_wait_read<1>();  // the store issued two chunks ago has read this buffer
-                        __syncwarp();
-                        uint8_t *sb = stg + sbuf * 2048;
-#pragma unroll
-                        for (int i = 0; i < 4; i++)
-                            *reinterpret_cast<uint4 *>(sb + lane * 64 + ((i ^ ((lane >> 1) & 3)) << 4)) =
-                                make_uint4(q[4 * i], q[4 * i + 1], q[4 * i + 2], q[4 * i + 3]);
+                        // y pass: TMA store of the 32 rows x 32 columns (64-byte swizzle of the
+                        // store map; the map clips rows and columns outside the volume).
                         fence_proxy_async_smem();
                         __syncwarp();
-                        // Every chunk commits exactly one bulk group (an empty one when the
-                        // chunk lies outside the volume), so that bulk_wait_read<1> above always
-                        // covers the store that last read the buffer being refilled.
                         if (lane == 0) {
-                            if (xb < c.nx && at * kTM + quad * 32 < c.A)
-                                tma_store_3d(c.out_map, sb, (int) xb, at * kTM + quad * 32, c.oth);
+                            tma_store_3d(c.out_map, stg, (int) xb, a0, c.oth);
                             bulk_commit();
                         }
-                        sbuf ^= 1;
                     }
                 }
-                tc_fence_before();
-                __syncwarp();
-                if (lane == 0) mbar_arrive(&tempty[d]);
             }
         }
     }
@@ -648,6 +692,7 @@ template <typename S, int FMT, class Sched>
 __global__ void __launch_bounds__(kXThreads, 1)
 tc_contig_kernel(const __grid_constant__ CUtensorMap tmap, const __grid_constant__ ContigLaunch<Sched> p) {
     const PassTaps &tp = p.taps;
+    pass_prepare();
     extern __shared__ uint8_t smem_raw[];
     const uint32_t raw = smem_u32(smem_raw);
     uint8_t *smem = smem_raw + (((raw + 1023) & ~1023u) - raw);
@@ -688,6 +733,7 @@ tc_contig_kernel(const __grid_constant__ CUtensorMap tmap, const __grid_constant
     tc_fence_after();
     const uint32_t tmem = *tmem_slot;
 
+    pass_wait();
     if (warp == 0 && lane == 0) {
         int64_t tl = 0;
         typename Sched::Cursor cc, cp;  // current tile, L2-prefetched tile
@@ -870,6 +916,7 @@ template <typename S, int FMT>
 __global__ void __launch_bounds__(kXtThreads, 1)
 tc_contig_t_kernel(const __grid_constant__ CUtensorMap tmap, const __grid_constant__ ContigLaunch<OneVolumeContigT> p) {
     const PassTaps &tp = p.taps;
+    pass_prepare();
     extern __shared__ uint8_t smem_raw[];
     const uint32_t raw = smem_u32(smem_raw);
     uint8_t *ring = smem_raw + (((raw + 1023) & ~1023u) - raw);
@@ -906,13 +953,14 @@ tc_contig_t_kernel(const __grid_constant__ CUtensorMap tmap, const __grid_consta
     const uint32_t tmem = *tmem_slot;
     if (warp >= 2) {
         // Tt^T: lane o holds x output o, K element j the tap j - o - RA + R.
-        toeplitz_to_tmem(tmem + kAcc, ring, tp, warp & 3, (warp - 2) >> 2, lane, tp.radius - tp.ra);
+        toeplitz_to_tmem(tmem + kAcc, ring, tp, warp & 3, (warp - 2) >> 2, kXtEpiWarps / 4, lane, tp.radius - tp.ra);
     }
     fence_proxy_async_smem();  // the ring's first copies land on the staged taps
     tc_fence_before();
     __syncthreads();
     tc_fence_after();
 
+    pass_wait();
     if (warp == 0 && lane == 0) {
         int64_t tl = 0;
         for (int64_t g = blockIdx.x; g < total; g += gridDim.x, tl++) {
@@ -1035,8 +1083,6 @@ inline void fill_pass_taps(PassTaps &t, const float *kernel, int radius, int ra,
     t.kp = kp;
     t.kpa = (int) round_up(kp, 64);
     t.kcols = toeplitz_cols(kp);
-    t.nbox = kp > 256 ? 2 : 1;  // kp is a multiple of 16, so kp / 2 is a whole number of 8-row swizzle atoms
-    t.box_rows = kp / t.nbox;
     t.error_feedback = error_feedback ? 1 : 0;
     const float scale = is_bf16 ? 1.0f : 1024.0f;
     t.inv_scale = 1.0f / scale;

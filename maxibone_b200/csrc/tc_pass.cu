@@ -61,7 +61,7 @@ cudaError_t tc_strided(const S *in, S *out, int64_t nz, int64_t ny, int64_t nx, 
                        int radius, bool error_feedback, cudaStream_t st, const YzRows *in_rows, bool hi_only) {
     if (!axis_z) in_rows = nullptr;
     const bool is_bf16 = std::is_same<S, __nv_bfloat16>::value;
-    const int tn = strided_tn(radius), stages = kStridedStages;
+    const int tn = strided_tn(radius, hi_only);
     StridedLaunch<OneVolumeStrided> p{};
     fill_pass_taps(p.taps, kernel, radius, 0, (int) round_up(kTM + 2 * radius, 16), is_bf16, error_feedback, hi_only);
     OneVolumeStrided &sc = p.sched;
@@ -80,7 +80,7 @@ cudaError_t tc_strided(const S *in, S *out, int64_t nz, int64_t ny, int64_t nx, 
     const CUtensorMapDataType dt = is_bf16 ? CU_TENSOR_MAP_DATA_TYPE_BFLOAT16 : CU_TENSOR_MAP_DATA_TYPE_FLOAT16;
     const cuuint64_t dims[3] = {(cuuint64_t) nx, (cuuint64_t) ny, (cuuint64_t) nz};
     const cuuint64_t strides[2] = {(cuuint64_t) (nx * 2), (cuuint64_t) (nx * ny * 2)};
-    const cuuint32_t brows = (cuuint32_t) p.taps.box_rows;
+    const cuuint32_t brows = (cuuint32_t) kStridedRows;
     const cuuint32_t box[3] = {64u, axis_z ? 1u : brows, axis_z ? brows : 1u};
     const cuuint32_t estr[3] = {1, 1, 1};
     // z pass over [y][z][x] rows: dims (x, z, y), rows nx apart, y slabs nz_total * nx apart.
@@ -101,20 +101,17 @@ cudaError_t tc_strided(const S *in, S *out, int64_t nz, int64_t ny, int64_t nx, 
                             CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
         if (cr != CUDA_SUCCESS) return cudaErrorInvalidValue;
     }
-    if (2 * tn + 2 * p.taps.kcols > (int) kTmemColsStrided) return cudaErrorInvalidValue;
-    const int smem = strided_smem_bytes(p.taps.kp, tn, stages);
+    if (2 * tn + (hi_only ? 1 : 2) * p.taps.kcols > (int) kTmemColsStrided) return cudaErrorInvalidValue;
+    const int smem = strided_smem_bytes(p.taps.kp, tn);
     auto *kern = tn == 128 ? (axis_z ? tc_strided_kernel<S, true, 128, OneVolumeStrided>
                                      : tc_strided_kernel<S, false, 128, OneVolumeStrided>)
                            : (axis_z ? tc_strided_kernel<S, true, 64, OneVolumeStrided>
                                      : tc_strided_kernel<S, false, 64, OneVolumeStrided>);
-    cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
-    if (e != cudaSuccess) return e;
     int dev = 0, sms = 148;
     cudaGetDevice(&dev);
     cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
     const int64_t grid = std::min<int64_t>(sc.n_cols, sms);
-    kern<<<(unsigned) grid, kThreads, smem, st>>>(map, map_out, p);
-    return cudaGetLastError();
+    return launch_pass(kern, nz * ny * nx < kOverlapVoxels, grid, strided_threads(tn), smem, st, map, map_out, p);
 }
 
 template cudaError_t tc_strided<__nv_bfloat16>(const __nv_bfloat16 *, __nv_bfloat16 *, int64_t, int64_t, int64_t,
@@ -334,11 +331,8 @@ cudaError_t tc_yx(const S *in, S *out, const void *mask, int mask_fmt, bool fina
                                    : tc_yx_kernel<S, MAXI_MASK_U8, false, OneVolumeYx>)
                      : (final_pass ? tc_yx_kernel<S, MAXI_MASK_BITPACKED, true, OneVolumeYx>
                                    : tc_yx_kernel<S, MAXI_MASK_BITPACKED, false, OneVolumeYx>);
-    cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
-    if (e != cudaSuccess) return e;
     const int64_t grid = std::min<int64_t>(sc.n_tiles, sms);
-    kern<<<(unsigned) grid, kYxThreads, smem, st>>>(map, omap, p);
-    return cudaGetLastError();
+    return launch_pass(kern, nz * ny * nx < kOverlapVoxels, grid, kYxThreads, smem, st, map, omap, p);
 }
 
 template cudaError_t tc_yx<__nv_bfloat16>(const __nv_bfloat16 *, __nv_bfloat16 *, const void *, int, bool, uint16_t *,
@@ -385,14 +379,11 @@ static cudaError_t tc_contig_t(const S *in, S *out, const void *mask, int mask_f
     if (cr != CUDA_SUCCESS) return cudaErrorInvalidValue;
     const int smem = contig_t_smem_bytes(p.taps.kpa);
     auto *kern = mask_fmt == MAXI_MASK_U8 ? tc_contig_t_kernel<S, MAXI_MASK_U8> : tc_contig_t_kernel<S, MAXI_MASK_BITPACKED>;
-    cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
-    if (e != cudaSuccess) return e;
     int dev = 0, sms = 148;
     cudaGetDevice(&dev);
     cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
     const int64_t grid = std::min<int64_t>(sc.n_tiles, sms);
-    kern<<<(unsigned) grid, kXtThreads, smem, st>>>(map, p);
-    return cudaGetLastError();
+    return launch_pass(kern, nz * ny * nx < kOverlapVoxels, grid, kXtThreads, smem, st, map, p);
 }
 
 template <typename S>
@@ -435,14 +426,11 @@ cudaError_t tc_contig(const S *in, S *out, const void *mask, int mask_fmt, bool 
     const int smem = contig_smem_bytes_tc(p.taps.kp, p.taps.kpa);
     auto *kern = mask_fmt == MAXI_MASK_U8 ? tc_contig_kernel<S, MAXI_MASK_U8, OneVolumeContig>
                                           : tc_contig_kernel<S, MAXI_MASK_BITPACKED, OneVolumeContig>;
-    cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
-    if (e != cudaSuccess) return e;
     int dev = 0, sms = 148;
     cudaGetDevice(&dev);
     cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
     const int64_t grid = std::min<int64_t>(sc.n_tiles, sms);
-    kern<<<(unsigned) grid, kXThreads, smem, st>>>(map, p);
-    return cudaGetLastError();
+    return launch_pass(kern, nz * ny * nx < kOverlapVoxels, grid, kXThreads, smem, st, map, p);
 }
 
 template cudaError_t tc_contig<__nv_bfloat16>(const __nv_bfloat16 *, __nv_bfloat16 *, const void *, int, bool,

@@ -167,7 +167,7 @@ struct ManyVolumesYx {
         }
         const TcVol &vol = vols[cur.v];
         YxTile t;
-        t.in = &vol.map[1][in_buf];
+        t.in = &vol.yxin[in_buf];
         t.out = &vol.yxrows[in_buf ^ 1];
         t.mask = vol.mask;
         t.out_u16 = vol.out_u16;
@@ -203,6 +203,7 @@ __global__ void __launch_bounds__(kYxThreads, 1)
 tc_yx_kernel(const __grid_constant__ CUtensorMap tmap, const __grid_constant__ CUtensorMap omap,
              const __grid_constant__ YxLaunch<Sched> p) {
     const PassTaps &tp = p.t;
+    pass_prepare();
     extern __shared__ uint8_t smem_raw[];
     const uint32_t raw = smem_u32(smem_raw);
     uint8_t *smem = smem_raw + (((raw + 1023) & ~1023u) - raw);
@@ -264,6 +265,7 @@ tc_yx_kernel(const __grid_constant__ CUtensorMap tmap, const __grid_constant__ C
     tc_fence_after();
     const uint32_t tmem = *tmem_slot;
 
+    pass_wait();
     if (warp == 0 && lane == 0) {
         // TMA producer: one F tile (nch boxes) per ring stage; L2 prefetch ahead.
         // The stage and its phase advance incrementally (the ring depth is a
