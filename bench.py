@@ -1014,8 +1014,9 @@ def main():
     achieved = b_alg * vox_local / (rep_ms / 1e3) / 1e9
     fused = bool(path & _lib.PATH_FUSED_YX)
     per_voxel_traffic = NCU_BYTES_PER_VOXEL_REP.get((args.field, "fused" if fused else "separate"))
+    # init: the uint8 mask read and packed; the FP32 form's first z pass reads the packed mask itself.
     kernel_bytes = {"z": 2 * s, "y": 2 * s, "x": 2 * s + 0.125, "x_final": s + 0.125 + 2, "yx": 2 * s + 0.125,
-                    "init": 0.125 + s}
+                    "init": 1.125 + (0 if args.field == "f32" else s)}
     per_kernel = {}
     for kind, (k_ms, k_n) in prof.items():
         if kind in kernel_bytes:

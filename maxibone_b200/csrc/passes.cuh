@@ -423,8 +423,8 @@ __device__ __forceinline__ void store_lit8(S *dst, uint32_t a, uint32_t b) {
 // The initial field of a mask and, from a uint8 mask, the packed mask with it, in one pass
 // over the mask: a thread takes 8 voxels (8 mask bytes or one byte of a packed word), so every
 // access of a warp is contiguous, and four such groups at a time.  Memory-bound: 1024^3 to
-// BF16 from bits 0.37 ms (2.1 GB written), before (a voxel per thread and step) 0.96 ms; from
-// bytes 0.51 ms, before 0.19 + 0.96 ms in two kernels.  `field` 16-byte and a uint8 mask 8-byte
+// BF16 from bits 0.37 ms (2.1 GB written), before (a voxel per thread and step) 0.96 ms; 256 x
+// 512 x 768 from bytes, with the packed mask, 0.053 ms, before 0.101 in two kernels.  `field` 16-byte and a uint8 mask 8-byte
 // aligned.
 template <typename S, int MASK_FMT>
 __global__ void __launch_bounds__(256)
