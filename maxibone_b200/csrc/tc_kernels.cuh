@@ -438,8 +438,10 @@ template <class Sched> struct ContigLaunch {
 // The passes are launched with programmatic stream serialization: a pass's blocks come up, with
 // barriers, tensor memory and the Toeplitz matrix, on the SMs that the pass before has left, and
 // touch the field only after pass_wait(), when that pass is complete and its writes are visible.
-// Every block waits, so a pass that is complete has all earlier ones behind it.  Without the
-// launch attribute both instructions do nothing.  It pays for one volume of fewer than
+// Every block waits, so a pass that is complete has all earlier ones behind it.  A block lets its
+// dependents come up (pass_prepare()) only once it holds its tensor memory: a dependent that took
+// the columns first would keep them until this pass is complete, which would then never be.
+// Without the launch attribute both instructions do nothing.  It pays for one volume of fewer than
 // kOverlapVoxels (20 repetitions of 200 x 344 x 456: 1714 -> 1653 us, four of 256 x 512 x 768
 // at radius 128: 1726 -> 1673); ten of 1024^3 take 21.58 ms without it and 21.80 with it, a batch
 // of 16 volumes 7.28 and 7.33 ms.
@@ -476,7 +478,6 @@ tc_strided_kernel(const __grid_constant__ CUtensorMap tmap, const __grid_constan
     constexpr int kEpiWarps = strided_epi_warps(TN);
     const PassTaps &tp = p.taps;
     const int stages = strided_stages(tp.kp);
-    pass_prepare();
     extern __shared__ uint8_t smem_raw[];
     const uint32_t raw = smem_u32(smem_raw);
     uint8_t *ring = smem_raw + (((raw + 1023) & ~1023u) - raw);
@@ -514,6 +515,7 @@ tc_strided_kernel(const __grid_constant__ CUtensorMap tmap, const __grid_constan
     __syncthreads();
     tc_fence_after();
     const uint32_t tmem = *tmem_slot;
+    pass_prepare();
     if (warp >= 2) {
         toeplitz_to_tmem(tmem + 2 * TN, ring, tp, warp & 3, (warp - 2) >> 2, kEpiWarps / 4, lane, 0);
     }
@@ -692,7 +694,6 @@ template <typename S, int FMT, class Sched>
 __global__ void __launch_bounds__(kXThreads, 1)
 tc_contig_kernel(const __grid_constant__ CUtensorMap tmap, const __grid_constant__ ContigLaunch<Sched> p) {
     const PassTaps &tp = p.taps;
-    pass_prepare();
     extern __shared__ uint8_t smem_raw[];
     const uint32_t raw = smem_u32(smem_raw);
     uint8_t *smem = smem_raw + (((raw + 1023) & ~1023u) - raw);
@@ -732,6 +733,7 @@ tc_contig_kernel(const __grid_constant__ CUtensorMap tmap, const __grid_constant
     __syncthreads();
     tc_fence_after();
     const uint32_t tmem = *tmem_slot;
+    pass_prepare();
 
     pass_wait();
     if (warp == 0 && lane == 0) {
@@ -916,7 +918,6 @@ template <typename S, int FMT>
 __global__ void __launch_bounds__(kXtThreads, 1)
 tc_contig_t_kernel(const __grid_constant__ CUtensorMap tmap, const __grid_constant__ ContigLaunch<OneVolumeContigT> p) {
     const PassTaps &tp = p.taps;
-    pass_prepare();
     extern __shared__ uint8_t smem_raw[];
     const uint32_t raw = smem_u32(smem_raw);
     uint8_t *ring = smem_raw + (((raw + 1023) & ~1023u) - raw);
@@ -951,6 +952,7 @@ tc_contig_t_kernel(const __grid_constant__ CUtensorMap tmap, const __grid_consta
     __syncthreads();
     tc_fence_after();
     const uint32_t tmem = *tmem_slot;
+    pass_prepare();
     if (warp >= 2) {
         // Tt^T: lane o holds x output o, K element j the tap j - o - RA + R.
         toeplitz_to_tmem(tmem + kAcc, ring, tp, warp & 3, (warp - 2) >> 2, kXtEpiWarps / 4, lane, tp.radius - tp.ra);

@@ -203,7 +203,6 @@ __global__ void __launch_bounds__(kYxThreads, 1)
 tc_yx_kernel(const __grid_constant__ CUtensorMap tmap, const __grid_constant__ CUtensorMap omap,
              const __grid_constant__ YxLaunch<Sched> p) {
     const PassTaps &tp = p.t;
-    pass_prepare();
     extern __shared__ uint8_t smem_raw[];
     const uint32_t raw = smem_u32(smem_raw);
     uint8_t *smem = smem_raw + (((raw + 1023) & ~1023u) - raw);
@@ -264,6 +263,7 @@ tc_yx_kernel(const __grid_constant__ CUtensorMap tmap, const __grid_constant__ C
     __syncthreads();
     tc_fence_after();
     const uint32_t tmem = *tmem_slot;
+    pass_prepare();
 
     pass_wait();
     if (warp == 0 && lane == 0) {
