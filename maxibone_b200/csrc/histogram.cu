@@ -43,6 +43,7 @@
 
 #include "common.cuh"
 #include "host_util.h"
+#include "launch.cuh"
 #include "scratch.h"
 
 namespace maxi {
@@ -898,7 +899,7 @@ int axis_launches(const uint16_t *voxels, int64_t nzl, int64_t Ny, int Nx, int64
     const bool exact = !vm.T;
     auto launch = [&](auto kernel, int64_t grid, int threads, int cells, auto... args) {
         const int smem = cells * (int) sizeof(uint32_t);
-        cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
+        cudaError_t e = allow_dynamic_smem(kernel, smem);
         if (e != cudaSuccess) return set_cuda_error(e, "axis histograms set-up");
         kernel<<<(unsigned) grid, threads, smem, st>>>(args...);
         return (int) MAXI_OK;

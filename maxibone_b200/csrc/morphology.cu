@@ -39,6 +39,7 @@
 // from radius 9 on: 1010 against 1074 us at r = 16 (twice the warps).
 #include "common.cuh"
 #include "host_util.h"
+#include "launch.cuh"
 #include "scratch.h"
 
 namespace maxi {
@@ -347,7 +348,7 @@ int morph_kernel(int radius, void (**kernel)(const uint32_t *, uint32_t *, const
     default: *kernel = morph_partials<DILATE, 32>; break;
     }
     int dev = 0, sms = 148, per_sm = 1;
-    cudaError_t e = cudaFuncSetAttribute(*kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, bucket_smem(radius));
+    cudaError_t e = allow_dynamic_smem(*kernel, bucket_smem(radius));
     if (e == cudaSuccess)
         e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, *kernel, kMorphThreads, bucket_smem(radius));
     if (e != cudaSuccess) return set_cuda_error(e, "morphology set-up");

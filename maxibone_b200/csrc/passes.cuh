@@ -24,17 +24,17 @@
 #pragma once
 
 #include "common.cuh"
+#include "launch.cuh"
 
 namespace maxi {
 
 template <int R> struct Taps { float k[2 * R + 1]; };
 
-// Programmatic dependent launch: the next pass's blocks may take free SM slots at once and
-// wait in pass_begin() until this pass is complete and its writes are visible.  Without the
-// launch attribute both instructions do nothing.
+// The head of an overlapped launch (launch.cuh): the next pass's blocks may take free SM slots at
+// once, and wait here until this pass is complete.
 __device__ __forceinline__ void pass_begin() {
-    asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
-    asm volatile("griddepcontrol.wait;" ::: "memory");
+    pass_prepare();
+    pass_wait();
 }
 
 // ---- strided (z / y) pass -------------------------------------------------

@@ -32,23 +32,6 @@ StreamShape stream_shape(int64_t outer, int64_t A, int64_t I, int tile, int chun
     return s;
 }
 
-template <typename... P, typename... Args>
-cudaError_t launch_pass(void (*kernel)(P...), int64_t blocks, int threads, int smem, cudaStream_t st, Args... args) {
-    cudaError_t e = set_smem(kernel, smem);
-    if (e != cudaSuccess) return e;
-    cudaLaunchAttribute attr{};
-    attr.id = cudaLaunchAttributeProgrammaticStreamSerialization;
-    attr.val.programmaticStreamSerializationAllowed = 1;
-    cudaLaunchConfig_t cfg{};
-    cfg.gridDim = dim3((unsigned) blocks);
-    cfg.blockDim = dim3(threads);
-    cfg.dynamicSmemBytes = smem;
-    cfg.stream = st;
-    cfg.attrs = &attr;
-    cfg.numAttrs = 1;
-    return cudaLaunchKernelEx(&cfg, kernel, args...);
-}
-
 bool aligned(const void *p, uintptr_t to) { return reinterpret_cast<uintptr_t>(p) % to == 0; }
 
 // z (outer 1, axis z) or y (outer z, axis y) pass; `mask`: read the field from it instead.
@@ -58,7 +41,7 @@ cudaError_t axis_pass(const float *in, const uint32_t *mask, float *out, int64_t
     const bool al = I % 4 == 0 && aligned(in, 16) && aligned(out, 16);
     auto kernel = mask ? (al ? stream_axis_pass<true, true> : stream_axis_pass<true, false>)
                        : (al ? stream_axis_pass<false, true> : stream_axis_pass<false, false>);
-    return launch_pass(kernel, outer * s.col_tiles * s.segments, kStreamThreads, s.ring * kStreamRow, st, in, mask, out, s, taps);
+    return launch_pass(kernel, true, outer * s.col_tiles * s.segments, kStreamThreads, s.ring * kStreamRow, st, in, mask, out, s, taps);
 }
 
 // The tile form of the x pass (contig_pass): 16-byte copies and unrolled taps.
@@ -66,7 +49,7 @@ template <int R, int MASK_FMT, bool FINAL>
 cudaError_t x_tile_pass(const float *in, float *out, const void *mask, uint16_t *out_u16, float *field_out,
                         int64_t rows, int64_t nx, const float *kernel, cudaStream_t st) {
     const int64_t xt = ceil_div(nx, kConTX);
-    return launch_pass(contig_pass<R, float, MASK_FMT, FINAL>, xt * ceil_div(rows, kConTR), kConThreads,
+    return launch_pass(contig_pass<R, float, MASK_FMT, FINAL>, true, xt * ceil_div(rows, kConTR), kConThreads,
                        contig_smem_bytes<R>(), st, in, out, mask, out_u16, field_out, rows, nx, xt,
                        make_taps<R>(kernel, R));
 }
@@ -93,7 +76,7 @@ cudaError_t x_pass(const float *in, float *out, const void *mask, uint16_t *out_
         }
     const StreamShape s = stream_shape(1, nx, rows, kStreamRowsX, kStreamChunkX, 32, radius);
     const int smem = kStreamRowsX * stream_x_pitch(s.ring) * 4 + kStreamMaskBytes;
-    return launch_pass(stream_x_pass<MASK_FMT, FINAL>, s.col_tiles * s.segments, kStreamThreads, smem, st, in, out,
+    return launch_pass(stream_x_pass<MASK_FMT, FINAL>, true, s.col_tiles * s.segments, kStreamThreads, smem, st, in, out,
                        mask, out_u16, field_out, s, taps);
 }
 

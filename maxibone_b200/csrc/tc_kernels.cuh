@@ -67,6 +67,7 @@
 #include <cudaTypedefs.h>
 
 #include "host_util.h"
+#include "launch.cuh"
 #include "tc_batch.h"
 #include "tc_common.cuh"
 #include "tc_pass.h"
@@ -437,36 +438,13 @@ template <class Sched> struct ContigLaunch {
 
 // The passes are launched with programmatic stream serialization: a pass's blocks come up, with
 // barriers, tensor memory and the Toeplitz matrix, on the SMs that the pass before has left, and
-// touch the field only after pass_wait(), when that pass is complete and its writes are visible.
-// Every block waits, so a pass that is complete has all earlier ones behind it.  A block lets its
-// dependents come up (pass_prepare()) only once it holds its tensor memory: a dependent that took
-// the columns first would keep them until this pass is complete, which would then never be.
-// Without the launch attribute both instructions do nothing.  It pays for one volume of fewer than
+// touch the field only after pass_wait().  A block lets its dependents come up (pass_prepare())
+// only once it holds its tensor memory: a dependent that took the columns first would keep
+// them until this pass is complete, which would then never be.  It pays for one volume of fewer than
 // kOverlapVoxels (20 repetitions of 200 x 344 x 456: 1714 -> 1653 us, four of 256 x 512 x 768
 // at radius 128: 1726 -> 1673); ten of 1024^3 take 21.58 ms without it and 21.80 with it, a batch
 // of 16 volumes 7.28 and 7.33 ms.
-__device__ __forceinline__ void pass_prepare() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
-__device__ __forceinline__ void pass_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
-
 constexpr int64_t kOverlapVoxels = int64_t(1) << 28;
-
-template <typename... Params, typename... Args>
-cudaError_t launch_pass(void (*kernel)(Params...), bool overlap, int64_t grid, int threads, int smem, cudaStream_t st,
-                        const Args &...args) {
-    cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
-    if (e != cudaSuccess) return e;
-    cudaLaunchAttribute attr{};
-    attr.id = cudaLaunchAttributeProgrammaticStreamSerialization;
-    attr.val.programmaticStreamSerializationAllowed = 1;
-    cudaLaunchConfig_t cfg{};
-    cfg.gridDim = dim3((unsigned) grid);
-    cfg.blockDim = dim3((unsigned) threads);
-    cfg.dynamicSmemBytes = (size_t) smem;
-    cfg.stream = st;
-    cfg.attrs = &attr;
-    cfg.numAttrs = overlap ? 1 : 0;
-    return cudaLaunchKernelEx(&cfg, kernel, args...);
-}
 
 // ---- z / y passes ------------------------------------------------------------------
 

@@ -31,12 +31,6 @@ static Taps<R> make_taps(const float *kernel, int radius) {
     return t;
 }
 
-template <typename F>
-static cudaError_t set_smem(F *f, int bytes) {
-    if (bytes <= 48 * 1024) return cudaSuccess;
-    return cudaFuncSetAttribute(f, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes);
-}
-
 template <typename S>
 cudaError_t launch_init_field(const void *mask, int mask_fmt, uint32_t *packed, S *field, int64_t n, cudaStream_t st) {
     const int64_t blocks = std::min<int64_t>(ceil_div(n, 256 * 8), 148 * 32);
@@ -65,14 +59,14 @@ static cudaError_t run_unrolled(const Volume &v, const void *mask, int mask_fmt,
     const int str_smem = strided_smem_bytes<R>();
     const int con_smem = contig_smem_bytes<R>();
     auto *zy = strided_pass<R, S, EF>;
-    cudaError_t e = set_smem(zy, str_smem);
+    cudaError_t e = allow_dynamic_smem(zy, str_smem);
     if (e != cudaSuccess) return e;
     auto *xu8 = contig_pass<R, S, MAXI_MASK_U8, false, EF>;
     auto *xu8f = contig_pass<R, S, MAXI_MASK_U8, true, EF>;
     auto *xbp = contig_pass<R, S, MAXI_MASK_BITPACKED, false, EF>;
     auto *xbpf = contig_pass<R, S, MAXI_MASK_BITPACKED, true, EF>;
     for (auto *f : {xu8, xu8f, xbp, xbpf})
-        if ((e = set_smem(f, con_smem)) != cudaSuccess) return e;
+        if ((e = allow_dynamic_smem(f, con_smem)) != cudaSuccess) return e;
     auto *xpass = mask_fmt == MAXI_MASK_U8 ? xu8 : xbp;
     auto *xfinal = mask_fmt == MAXI_MASK_U8 ? xu8f : xbpf;
 
