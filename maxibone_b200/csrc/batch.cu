@@ -34,6 +34,7 @@
 
 #include "host_util.h"
 #include "tc_batch.h"
+#include "scratch.h"
 #include "unrolled.h"
 
 extern "C" int64_t maxi_diffusion_workspace_size(int64_t nz, int64_t ny, int64_t nx, int32_t field_type);
@@ -515,7 +516,7 @@ int maxi_batch_plan_create(const maxi_volume *volumes, int64_t n_volumes, int32_
         total += round_up(maxi_diffusion_workspace_size(bv.v.nz, bv.v.ny, bv.v.nx, bv.run_type), 1024);
         p->vols.push_back(bv);
     }
-    if (cudaMalloc(&p->d_ws, total) != cudaSuccess) {
+    if (with_room([&] { return cudaMalloc(&p->d_ws, total); }) != cudaSuccess) {
         cudaGetLastError();
         destroy_plan(p);
         return set_error(MAXI_ERR_OUT_OF_MEMORY, "could not allocate %lld bytes of batch workspace", (long long) total);

@@ -193,7 +193,7 @@ static int device_cache(DeviceCache **out) {
 static int cache_reserve(DeviceCache *c, int64_t bytes) {
     if (c->bytes >= bytes) return MAXI_OK;
     cache_drop(c);
-    if (cudaMalloc(&c->buf, bytes) != cudaSuccess) {
+    if (with_room([&] { return cudaMalloc(&c->buf, bytes); }) != cudaSuccess) {
         cudaGetLastError();
         c->buf = nullptr;
         return set_error(MAXI_ERR_OUT_OF_MEMORY, "could not allocate %lld bytes on the device", (long long) bytes);
@@ -344,7 +344,7 @@ int maxi::diffusion_device_shrinking(const void *mask, int32_t mask_format, int6
             return set_error(MAXI_ERR_INVALID_ARGUMENT, "workspace of %lld bytes is smaller than the %lld needed",
                              (long long) workspace_bytes, (long long) need);
         if (!ws) {
-            if (cudaMallocAsync(reinterpret_cast<void **>(&ws), need, st) != cudaSuccess) {
+            if (with_room([&] { return cudaMallocAsync(reinterpret_cast<void **>(&ws), need, st); }) != cudaSuccess) {
                 cudaGetLastError();
                 return set_error(MAXI_ERR_OUT_OF_MEMORY, "could not allocate %lld bytes of device workspace",
                                  (long long) need);

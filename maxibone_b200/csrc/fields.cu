@@ -38,6 +38,7 @@
 #include <vector>
 
 #include "common.cuh"
+#include "host_copy.h"
 #include "host_util.h"
 #include "scratch.h"
 
@@ -357,12 +358,11 @@ extern "C" int maxi_combine_fields(const uint16_t *gauss, const uint16_t *edt, i
     bool any_outside = false, any_inside = false;
     cylinder_intervals(ny, nx, inside, any_outside, any_inside);
 
-    std::unique_lock<std::mutex> hold;
-    char *scratch = nullptr;
     const size_t iv_bytes = (size_t) ny * sizeof(int2);
-    if ((rc = acquire_scratch(256 + iv_bytes, hold, &scratch, "field combination"))) return rc;
-    CombineStats *d_st = reinterpret_cast<CombineStats *>(scratch);
-    int2 *d_iv = reinterpret_cast<int2 *>(scratch + 256);
+    SpareBuffer scratch;
+    if ((rc = scratch.take(256 + iv_bytes, st, "field combination"))) return rc;
+    CombineStats *d_st = reinterpret_cast<CombineStats *>(scratch.data());
+    int2 *d_iv = reinterpret_cast<int2 *>(scratch.data() + 256);
     const bool aligned = ((reinterpret_cast<uintptr_t>(gauss) | reinterpret_cast<uintptr_t>(edt) |
                            reinterpret_cast<uintptr_t>(output)) & 15) == 0;
     const bool vec = nx % 8 == 0 && aligned;
@@ -374,7 +374,9 @@ extern "C" int maxi_combine_fields(const uint16_t *gauss, const uint16_t *edt, i
     while (lanes < 32 && lanes * (vec ? 8 : 1) < nx) lanes *= 2;
     const unsigned grid_flat = (unsigned) std::min<int64_t>(ceil_div(ceil_div(rows * nx, 8), threads), (int64_t) sms * 16);
     const unsigned grid = (unsigned) std::min<int64_t>(ceil_div(rows * lanes, threads), (int64_t) sms * 16);
-    CombineStats h{};
+    CombineStats pageable{};
+    const StagingBuffer staging;
+    CombineStats &h = staging.data() ? *static_cast<CombineStats *>(staging.data()) : pageable;
     cudaError_t e = cudaMemsetAsync(d_st, 0, sizeof(CombineStats), st);
     if (e == cudaSuccess) e = cudaMemcpyAsync(d_iv, inside.data(), iv_bytes, cudaMemcpyHostToDevice, st);
     if (e == cudaSuccess) {
@@ -387,7 +389,7 @@ extern "C" int maxi_combine_fields(const uint16_t *gauss, const uint16_t *edt, i
         e = cudaGetLastError();
     }
     if (e == cudaSuccess) e = cudaMemcpyAsync(&h, d_st, sizeof(h), cudaMemcpyDeviceToHost, st);
-    cudaError_t e2 = cudaStreamSynchronize(st);  // the scratch and the host intervals are free after it
+    cudaError_t e2 = scratch.give_back();  // waits for the stream: the host intervals are free after it
     if (e == cudaSuccess) e = e2;
     if (e != cudaSuccess) return set_cuda_error(e, "combine_fields");
     if (h.gmax == 0 || h.emax == 0)

@@ -1058,19 +1058,18 @@ extern "C" int maxi_field_histogram(const uint16_t *voxels, int64_t nZ, int64_t 
     const size_t o_x = t.add(xmap.data(), xmap.size());
     const size_t tables = (t.host.size() * sizeof(uint32_t) + 255) / 256 * 256;
     FieldPlan f = field_plan(nZ, nY, nX, field_bins, voxel_bins, tables);
-    std::unique_lock<std::mutex> lock;  // holds the scratch until the launches are done
-    uint8_t *scratch = nullptr;
-    rc = acquire_scratch(f.bytes, lock, &scratch, "histogram");
+    SpareBuffer scratch;
+    rc = scratch.take(f.bytes, st, "histogram");
     if (rc == MAXI_ERR_OUT_OF_MEMORY && f.partitioned) {  // the direct form needs the tables alone
         clear_error();
-        if (lock) lock.unlock();
         f.partitioned = false;
-        rc = acquire_scratch(tables, lock, &scratch, "histogram");
+        rc = scratch.take(tables, st, "histogram");
     }
     if (rc) return rc;
-    cudaError_t e = cudaMemcpyAsync(scratch, t.host.data(), t.host.size() * sizeof(uint32_t), cudaMemcpyHostToDevice, st);
+    cudaError_t e =
+        cudaMemcpyAsync(scratch.data(), t.host.data(), t.host.size() * sizeof(uint32_t), cudaMemcpyHostToDevice, st);
     if (e != cudaSuccess) return set_cuda_error(e, "histogram tables");
-    const uint32_t *dev = reinterpret_cast<const uint32_t *>(scratch);
+    const uint32_t *dev = reinterpret_cast<const uint32_t *>(scratch.data());
     if (!vT.empty()) vm.T = dev + o_vT;
     if (!fT.empty()) fm.T = dev + o_fT;
     const int32_t *zm = reinterpret_cast<const int32_t *>(dev + o_z);
@@ -1096,7 +1095,7 @@ extern "C" int maxi_field_histogram(const uint16_t *voxels, int64_t nZ, int64_t 
         a.voxel_bins = (int) voxel_bins;
         a.field_bins = (int) field_bins;
         a.bins = b;
-        rc = field_launches(f, a, scratch, nZ * nY, vec, st);
+        rc = field_launches(f, a, scratch.data(), nZ * nY, vec, st);
     } else {
         const unsigned grid = (unsigned) std::min<int64_t>(nZ * nY, (int64_t) sm_count() * 16);
         if (vec)
@@ -1106,8 +1105,11 @@ extern "C" int maxi_field_histogram(const uint16_t *voxels, int64_t nZ, int64_t 
             field_histogram_kernel<false><<<grid, 256, 0, st>>>(voxels, field, nZ, nY, (int) nX, ny, nx, y_start,
                                                                 (int) x_start, vm, fm, zm, ym, xm, b, voxel_bins);
     }
-    t.dev = nullptr;  // the scratch stays
-    return finish(t, st, rc, "field histogram");
+    e = rc == MAXI_OK ? cudaGetLastError() : cudaSuccess;
+    const cudaError_t e2 = scratch.give_back();  // waits for the stream: the host tables are free after it
+    if (rc) return rc;
+    if (e == cudaSuccess) e = e2;
+    return e == cudaSuccess ? MAXI_OK : set_cuda_error(e, "field histogram");
 }
 
 extern "C" int maxi_axis_histograms(const uint16_t *voxels, int64_t nz_block, int64_t Nz, int64_t Ny, int64_t Nx,

@@ -170,6 +170,12 @@ cudaError_t copy_to_host_staged(void *h_dst, const void *d_src, size_t n, cudaSt
     });
 }
 
+StagingBuffer::StagingBuffer() {
+    if (take_buffers(1, bufs_) != cudaSuccess) cudaGetLastError();
+}
+
+StagingBuffer::~StagingBuffer() { return_buffers(bufs_); }
+
 void release_staging_buffers() {
     std::vector<void *> bufs;
     {

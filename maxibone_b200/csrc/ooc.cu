@@ -41,6 +41,7 @@
 #include <functional>
 
 #include "host_util.h"
+#include "scratch.h"
 #include "unrolled.h"
 
 namespace maxi {
@@ -254,6 +255,7 @@ static int run_slabs(int64_t nz, int64_t ny, int64_t nx, int64_t slab_z, const f
         return set_error(MAXI_ERR_INVALID_ARGUMENT, "unknown field_type %d", field_type);
 
     size_t free_b = 0, total_b = 0;
+    free_spare_buffers();
     cudaMemGetInfo(&free_b, &total_b);
     const SlabPlan pl = full_plan(nz, ny, nx, slab_z, kernel_size, repititions, field_type, flags, device_budget(free_b),
                                   host_budget());
@@ -591,6 +593,7 @@ extern "C" int maxi_out_of_core_plan(int64_t nz, int64_t ny, int64_t nx, int64_t
     if (device_bytes <= 0) {
         if ((rc = require_device())) return rc;
         size_t free_b = 0, total_b = 0;
+        free_spare_buffers();
         cudaError_t e = cudaMemGetInfo(&free_b, &total_b);
         if (e != cudaSuccess) return set_cuda_error(e, "cudaMemGetInfo");
         device_bytes = device_budget(free_b);
