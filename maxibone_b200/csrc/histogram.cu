@@ -509,8 +509,9 @@ __device__ __forceinline__ int64_t isqrt64(int64_t n) {
 }
 
 // axis_histograms where the shared-memory forms below do not apply: every voxel adds to the
-// global bins, runs of equal keys once (x: every voxel).
-template <bool VEC8>
+// global bins, runs of equal keys once (x: every voxel).  RADIAL: the radial histogram alone, for
+// distances beyond ring_histograms.
+template <bool VEC8, bool RADIAL>
 __global__ void axis_histograms_direct(const uint16_t *__restrict__ voxels, int64_t nzl, int64_t Ny, int Nx,
                                        int64_t z_start, int64_t y_start, int x_start, BinMap vm, int64_t cy,
                                        int64_t cx, unsigned long long *__restrict__ x_bins,
@@ -539,7 +540,7 @@ __global__ void axis_histograms_direct(const uint16_t *__restrict__ voxels, int6
                 const int vb = x >= x_start ? bin_of(vm, v[j]) : -1;
                 long long rk = -1;
                 if (vb >= 0) {
-                    atomicAdd(x_bins + (int64_t) x * voxel_bins + vb, 1ull);
+                    if (!RADIAL) atomicAdd(x_bins + (int64_t) x * voxel_bins + vb, 1ull);
                     const int64_t r = isqrt64(dy2 + (x - cx) * (x - cx));
                     if (r < n_r) rk = r * voxel_bins + vb;
                 }
@@ -550,6 +551,7 @@ __global__ void axis_histograms_direct(const uint16_t *__restrict__ voxels, int6
                     r_key = rk;
                     r_run = 1;
                 }
+                if (RADIAL) continue;
                 if (vb == b_key) {
                     b_run++;
                 } else {
@@ -582,13 +584,14 @@ __device__ __forceinline__ void counters_flush(const uint32_t *c, int n, unsigne
 }
 
 // y_bins or z_bins: block (p, chunk) counts the rows row0(p), row0(p) + row_step, .. of one y
-// (or z), from row chunk * per on, in one shared histogram.  A warp per row.
+// (or z), from row chunk * per on, in one shared histogram.  A warp per row; SPLIT: several of them
+// per row, where the chunk has fewer rows than the block has warps.
 struct RowSets {
     int64_t sets, set_step, row_step, rows, first_row, per;  // per: rows of a chunk
     int64_t first_set;                                      // sets below are not counted
     unsigned long long *bins;                               // of set 0
 };
-template <bool VEC8, bool EXACT>
+template <bool VEC8, bool EXACT, bool SPLIT>
 __global__ void __launch_bounds__(256) row_set_histograms(const uint16_t *__restrict__ voxels, int Nx, int x_start,
                                                           BinMap vm, RowSets s, int voxel_bins) {
     extern __shared__ uint32_t counters[];
@@ -600,17 +603,21 @@ __global__ void __launch_bounds__(256) row_set_histograms(const uint16_t *__rest
         const int b = bin_of<EXACT>(vm, v);
         if (b >= 0) atomicAdd(counters + b, 1u);
     };
-    for (int64_t i = s.first_row + chunk * s.per + (threadIdx.x >> 5); i < end; i += blockDim.x >> 5) {
+    const int64_t begin = s.first_row + chunk * s.per;
+    int split = 0;  // 2^split warps to a row
+    while (SPLIT && split < 3 && (end - begin) << (split + 1) <= 8) split++;
+    const int warp = threadIdx.x >> 5, share = SPLIT ? warp & ((1 << split) - 1) : 0, shares = 1 << split;
+    for (int64_t i = begin + (warp >> split); i < end; i += 8 >> split) {
         const uint16_t *row = voxels + (set * s.set_step + i * s.row_step) * Nx;
         if (VEC8) {
             // Up to x_first one voxel per lane, then two loads of 8 ahead of their counting.
             const int x_first = (x_start + kVec - 1) / kVec * kVec;
-            if (x_start + lane < x_first) count(__ldcs(row + x_start + lane));
-            for (int x = x_first + lane * kVec; x < Nx; x += 64 * kVec) {
+            if (share == 0 && x_start + lane < x_first) count(__ldcs(row + x_start + lane));
+            for (int x = x_first + (lane + 32 * share) * kVec; x < Nx; x += 64 * shares * kVec) {
                 int v[kVec], w[kVec];
-                const bool second = x + 32 * kVec < Nx;
+                const bool second = x + 32 * shares * kVec < Nx;
                 load_row8(row + x, v);
-                if (second) load_row8(row + x + 32 * kVec, w);
+                if (second) load_row8(row + x + 32 * shares * kVec, w);
 #pragma unroll
                 for (int j = 0; j < kVec; j++) count(v[j]);
                 if (second)
@@ -618,7 +625,7 @@ __global__ void __launch_bounds__(256) row_set_histograms(const uint16_t *__rest
                     for (int j = 0; j < kVec; j++) count(w[j]);
             }
         } else {
-            for (int x = x_start + lane; x < Nx; x += 32 * kVec) {
+            for (int x = x_start + lane + 32 * kVec * share; x < Nx; x += 32 * kVec * shares) {
                 int v[kVec];
 #pragma unroll
                 for (int j = 0; j < kVec; j++) v[j] = x + 32 * j < Nx ? __ldcs(row + x + 32 * j) : -1;
@@ -685,47 +692,83 @@ __device__ __forceinline__ int isqrt32(int n) {
     return r;
 }
 
-// r_bins: block (ring, chunk) counts the pixels with ring * width <= r < (ring + 1) * width
-// over the planes of the chunk.  Eight lanes take a row: its pixels of the ring are at most
-// two x intervals (of about `width` each for most rows, hence eight), a lane per pixel, which
-// reads that pixel of every plane, eight ahead of their counting.  The outer, larger rings
-// start first.  Distances stay below 2^31 (the host checks).
-template <bool EXACT>
+// r_bins: block (ring, chunk, part) counts the pixels with ring * width <= r < (ring + 1) * width
+// over the planes of the chunk and, `parts` to a ring, every so many of its rows.  Eight lanes take
+// a row: its pixels of the ring are at most two x intervals (of about `width` each for most
+// rows, hence eight), a lane per pixel, which reads that pixel of every plane, eight ahead of
+// their counting.  SPLIT: where the ring's rows do not fill the block, eights of planes and then
+// more lanes go to a row, and of one or two planes a lane loads four pixels ahead.  Rows that the
+// ring meets only outside the volume are left out (a 2 x 40000 x 1000 block, 4096 bins: a ring's
+// blocks would walk 40000 rows for about 40; the call 790 us with both, 2450 without).  The outer,
+// larger rings start first.  Squared distances stay below 2^31 (the host checks).
+template <bool EXACT, bool SPLIT>
 __global__ void __launch_bounds__(1024) ring_histograms(const uint16_t *__restrict__ voxels, int64_t nzl, int Ny,
                                                         int Nx, int y_start, int x_start, BinMap vm, int cy, int cx,
-                                                        int rings, int width, int64_t per,
+                                                        int rings, int width, int64_t per, int parts,
                                                         unsigned long long *__restrict__ r_bins, int voxel_bins,
                                                         int n_r) {
     extern __shared__ uint32_t counters[];
     const int64_t chunks = (nzl + per - 1) / per;
-    const int ring = rings - 1 - (int) (blockIdx.x / chunks);
-    const int64_t z0 = blockIdx.x % chunks * per;
+    const int part = (int) (blockIdx.x % parts);
+    const int ring = rings - 1 - (int) (blockIdx.x / parts / chunks);
+    const int64_t z0 = blockIdx.x / parts % chunks * per;
     const int planes = (int) min(per, nzl - z0);
     const int r0 = ring * width, r1 = min(r0 + width, n_r);
     counters_clear(counters, (r1 - r0) * voxel_bins);
     const int64_t plane = (int64_t) Ny * Nx;
     const int inner = r0 * r0, outer = r1 * r1 - 1;  // squared distances inner .. outer
-    const int y_end = min(Ny - 1, cy + r1 - 1), lane = threadIdx.x & 7;
-    for (int y = max(y_start, cy - r1 + 1) + (threadIdx.x >> 3); y <= y_end; y += blockDim.x >> 3) {
+    // The rows' distances low .. reach from the centre: those at which the ring meets a column.
+    const int64_t widest = max(abs(x_start - cx), abs(Nx - 1 - cx)), nearest = max(0, max(x_start - cx, cx - (Nx - 1)));
+    const int low = inner > widest * widest ? isqrt32((int) (inner - widest * widest) - 1) + 1 : 0;
+    const int reach = outer >= nearest * nearest ? isqrt32((int) (outer - nearest * nearest)) : -1;
+    const int above = max(y_start, cy - reach), n_above = max(0, min(Ny - 1, cy - max(low, 1)) - above + 1);
+    const int below = max(y_start, cy + low), n_rows = n_above + max(0, min(Ny - 1, cy + reach) - below + 1);
+    // 2^lane_bits lanes to a row and an eighth of planes, 2^z_bits of these to a row.
+    const int rows = (n_rows + parts - 1) / parts;
+    int lane_bits = 3, z_bits = 0;
+    while (SPLIT && (8 << z_bits) < planes && rows << (lane_bits + z_bits + 1) <= 1024) z_bits++;
+    while (SPLIT && lane_bits < 8 && rows << (lane_bits + z_bits + 1) <= 1024) lane_bits++;
+    const int lane = threadIdx.x & ((1 << lane_bits) - 1), lanes = 1 << lane_bits;
+    const int z_first = SPLIT ? 8 * ((threadIdx.x >> lane_bits) & ((1 << z_bits) - 1)) : 0, z_step = 8 << z_bits;
+    const int slot = threadIdx.x >> (lane_bits + z_bits), step = 1024 >> (lane_bits + z_bits);
+    auto count = [&](uint32_t *c, int v) {
+        const int b = bin_of<EXACT>(vm, v);
+        if (b >= 0 && v >= 0) atomicAdd(c + b, 1u);
+    };
+    for (int i = part * step + slot; i < n_rows; i += parts * step) {
+        const int y = i < n_above ? above + i : below + (i - n_above);
         const int dy2 = (y - cy) * (y - cy);
         const int far = isqrt32(outer - dy2), near = dy2 >= inner ? 0 : isqrt32(inner - dy2 - 1) + 1;
         // right: cx + near .. cx + far; left: cx - far .. cx - max(near, 1)
         const int right = max(cx + near, x_start), n_right = max(0, min(cx + far, Nx - 1) - right + 1);
         const int left = max(cx - far, x_start), n_left = max(0, min(cx - max(near, 1), Nx - 1) - left + 1);
         const uint16_t *row = voxels + z0 * plane + (int64_t) y * Nx;
-        for (int k = lane; k < n_right + n_left; k += 8) {
-            const int x = k < n_right ? right + k : left + (k - n_right);
-            uint32_t *c = counters + (isqrt32(dy2 + (x - cx) * (x - cx)) - r0) * voxel_bins;
-            const uint16_t *p = row + x;
-            for (int z = 0; z < planes; z += 8, p += 8 * plane) {
+        const int n = n_right + n_left;
+        auto x_of = [&](int k) { return k < n_right ? right + k : left + (k - n_right); };
+        auto counters_of = [&](int x) { return counters + (isqrt32(dy2 + (x - cx) * (x - cx)) - r0) * voxel_bins; };
+        if (SPLIT && planes <= 2) {
+            for (int z = 0; z < planes; z++, row += plane) {
+                for (int k = lane; k < n; k += 4 * lanes) {
+                    int v[4];
+#pragma unroll
+                    for (int j = 0; j < 4; j++) v[j] = k + j * lanes < n ? __ldg(row + x_of(k + j * lanes)) : -1;
+#pragma unroll
+                    for (int j = 0; j < 4; j++)
+                        if (v[j] >= 0) count(counters_of(x_of(k + j * lanes)), v[j]);
+                }
+            }
+            continue;
+        }
+        for (int k = lane; k < n; k += lanes) {
+            const int x = x_of(k);
+            uint32_t *c = counters_of(x);
+            const uint16_t *p = row + x + z_first * plane;
+            for (int z = z_first; z < planes; z += z_step, p += z_step * plane) {
                 int v[8];
 #pragma unroll
                 for (int j = 0; j < 8; j++) v[j] = z + j < planes ? __ldg(p + j * plane) : -1;
 #pragma unroll
-                for (int j = 0; j < 8; j++) {
-                    const int b = bin_of<EXACT>(vm, v[j]);
-                    if (b >= 0 && v[j] >= 0) atomicAdd(c + b, 1u);
-                }
+                for (int j = 0; j < 8; j++) count(c, v[j]);
             }
         }
     }
@@ -844,35 +887,26 @@ int sm_count() {
     return sms;
 }
 
-// Device copy of host words laid out in 16-byte aligned segments.
-struct DeviceTables {
-    std::vector<uint32_t> host;
-    uint32_t *dev = nullptr;
+// Host words laid out in 16-byte aligned segments, for one copy to the device.
+struct HostTables {
+    std::vector<uint32_t> words;
     size_t add(const uint32_t *p, size_t n) {
-        const size_t at = host.size();
-        host.insert(host.end(), p, p + n);
-        host.resize((host.size() + 3) / 4 * 4, 0);
+        const size_t at = words.size();
+        words.insert(words.end(), p, p + n);
+        words.resize((words.size() + 3) / 4 * 4, 0);
         return at;
+    }
+    size_t bytes() const { return words.size() * sizeof(uint32_t); }
+    cudaError_t copy_to(void *dev, cudaStream_t st) const {
+        return cudaMemcpyAsync(dev, words.data(), bytes(), cudaMemcpyHostToDevice, st);
     }
 };
 
-int upload(DeviceTables &t, cudaStream_t st) {
-    const size_t bytes = t.host.size() * sizeof(uint32_t);
-    if (bytes == 0) return MAXI_OK;
-    if (cudaMallocAsync(reinterpret_cast<void **>(&t.dev), bytes, st) != cudaSuccess) {
-        cudaGetLastError();
-        t.dev = nullptr;
-        return set_error(MAXI_ERR_OUT_OF_MEMORY, "could not allocate %zu bytes of tables", bytes);
-    }
-    cudaError_t e = cudaMemcpyAsync(t.dev, t.host.data(), bytes, cudaMemcpyHostToDevice, st);
-    return e == cudaSuccess ? MAXI_OK : set_cuda_error(e, "histogram tables");
-}
-
-// Waits for the launch (the host tables must outlive their copy) and frees the device copy.
-int finish(DeviceTables &t, cudaStream_t st, int rc, const char *what) {
+// The status of a call whose launches gave `rc`; waits for `st`, as the host tables must outlive
+// their copy.
+int finish(SpareBuffer &scratch, cudaStream_t st, int rc, const char *what) {
     cudaError_t e = rc == MAXI_OK ? cudaGetLastError() : cudaSuccess;
-    cudaError_t e2 = cudaStreamSynchronize(st);
-    if (t.dev) cudaFreeAsync(t.dev, st);
+    const cudaError_t e2 = scratch.data() ? scratch.give_back() : cudaStreamSynchronize(st);
     if (rc != MAXI_OK) return rc;
     if (e == cudaSuccess) e = e2;
     return e == cudaSuccess ? MAXI_OK : set_cuda_error(e, what);
@@ -889,13 +923,14 @@ int axis_launches(const uint16_t *voxels, int64_t nzl, int64_t Ny, int Nx, int64
                   unsigned long long *zb, unsigned long long *rb, int voxel_bins, int64_t n_r, bool vec,
                   int64_t farthest, cudaStream_t st) {
     const int64_t sms = sm_count(), rows = nzl * Ny;
-    if (voxel_bins > kMaxSharedBins || rows * Nx < kAxisMinVoxels || farthest >= (1 << 15) || n_r >= (1 << 15)) {
+    auto direct = [&](auto kernel) {
         const unsigned grid = (unsigned) std::min<int64_t>(rows, sms * 16);
-        auto direct = vec ? axis_histograms_direct<true> : axis_histograms_direct<false>;
-        direct<<<grid, vec ? 128 : 256, 0, st>>>(voxels, nzl, Ny, Nx, z_start, y_start, x_start, vm, cy, cx, xb, yb, zb,
+        kernel<<<grid, vec ? 128 : 256, 0, st>>>(voxels, nzl, Ny, Nx, z_start, y_start, x_start, vm, cy, cx, xb, yb, zb,
                                                  rb, voxel_bins, n_r);
-        return MAXI_OK;
-    }
+        return (int) MAXI_OK;
+    };
+    if (voxel_bins > kMaxSharedBins || rows * Nx < kAxisMinVoxels)
+        return direct(vec ? axis_histograms_direct<true, false> : axis_histograms_direct<false, false>);
     const bool exact = !vm.T;
     auto launch = [&](auto kernel, int64_t grid, int threads, int cells, auto... args) {
         const int smem = cells * (int) sizeof(uint32_t);
@@ -911,8 +946,12 @@ int axis_launches(const uint16_t *voxels, int64_t nzl, int64_t Ny, int Nx, int64
         const int64_t chunks = std::max<int64_t>(1, std::min(ceil_div(sms * 8, counted), n / 16));
         const int64_t per = ceil_div(n, chunks);
         const RowSets s{sets, set_step, row_step, row_count, first_row, per, first_set, bins};
-        return launch(vec ? (exact ? row_set_histograms<true, true> : row_set_histograms<true, false>)
-                          : (exact ? row_set_histograms<false, true> : row_set_histograms<false, false>), counted * ceil_div(n, per), 256,
+        auto kernel = [&](auto split) {
+            constexpr bool S = decltype(split)::value;
+            return vec ? (exact ? row_set_histograms<true, true, S> : row_set_histograms<true, false, S>)
+                       : (exact ? row_set_histograms<false, true, S> : row_set_histograms<false, false, S>);
+        };
+        return launch(per < 8 ? kernel(std::true_type{}) : kernel(std::false_type{}), counted * ceil_div(n, per), 256,
                       voxel_bins, voxels, Nx, x_start, vm, s, voxel_bins);
     };
     int rc = row_sets(nzl, 0, Ny, 1, Ny, y_start, zb + z_start * voxel_bins);
@@ -927,14 +966,34 @@ int axis_launches(const uint16_t *voxels, int64_t nzl, int64_t Ny, int Nx, int64
                      : (exact ? strip_histograms<false, true> : strip_histograms<false, false>), strips * ceil_div(rows, x_per),
                 1024, strip * voxel_bins, voxels, rows, Ny, Nx, y_start, x_start, vm, strips, strip, x_per, xb, voxel_bins);
     if (rc) return rc;
-    // r: rings of as many radii as the counters allow; 16 planes per block.
+    // r: rings of as many radii as the counters allow, up to 64 (a wider row interval reads no
+    // fewer sectors), in chunks of 16 planes or more.  Few rings, of a volume with few bins or
+    // planes, are shared by several blocks, as long as a block has 8 pixels per counter that
+    // it clears and adds to the bins; if that leaves SMs idle, the rings get narrower.
+    // (1 x 4096 x 4096, 64 bins: 5510 us with 6 blocks of 512 radii, 169 now.)
     const int64_t radii = std::min<int64_t>(n_r, (int64_t) (1.4142136 * (double) farthest) + 2);
-    const int width = (int) std::min<int64_t>(radii, std::max(1, kBlockCells / voxel_bins));
-    const int rings = (int) ceil_div(radii, width);
-    const int64_t per = std::min<int64_t>(nzl, 16);
-    return launch(exact ? ring_histograms<true> : ring_histograms<false>, rings * ceil_div(nzl, per), 1024,
-                  width * voxel_bins, voxels, nzl, (int) Ny, Nx, (int) y_start, x_start, vm, (int) cy, (int) cx, rings,
-                  width, per, rb, voxel_bins, (int) n_r);
+    if (radii > 46340 - 64)  // squared distances of 2^31 in the last ring
+        return direct(vec ? axis_histograms_direct<true, true> : axis_histograms_direct<false, true>);
+    int64_t width = std::min<int64_t>({radii, 64, std::max(1, kBlockCells / voxel_bins)});
+    int64_t rings, chunks, parts;
+    for (;; width /= 2) {
+        rings = ceil_div(radii, width);
+        chunks = std::min(ceil_div(sms * 6, rings), ceil_div(nzl, 16));
+        const int64_t pixels = rows * Nx / (rings * chunks);
+        parts = std::max<int64_t>(1, std::min({ceil_div(sms * 6, rings * chunks), ceil_div(std::min(Ny, 2 * radii), 128),
+                                               pixels / (8 * width * voxel_bins)}));
+        if (rings * chunks * parts >= sms * 3 / 4 || width <= kVec) break;
+    }
+    const int64_t per = ceil_div(nzl, chunks);
+    // Rows that a ring of half the largest radius meets.
+    const double half = 0.5 * (double) radii, widest = (double) std::max(std::abs(x_start - cx), std::abs(Nx - 1 - cx));
+    const double low = std::sqrt(std::max(0.0, half * half - widest * widest));
+    const bool split = per <= 2 || 2.0 * (half + (double) width - low) < 64.0 || Ny < 64;
+    auto kernel = split ? (exact ? ring_histograms<true, true> : ring_histograms<false, true>)
+                        : (exact ? ring_histograms<true, false> : ring_histograms<false, false>);
+    return launch(kernel, rings * ceil_div(nzl, per) * parts, 1024, (int) width * voxel_bins, voxels, nzl, (int) Ny, Nx,
+                  (int) y_start, x_start, vm, (int) cy, (int) cx, (int) rings, (int) width, per, (int) parts, rb,
+                  voxel_bins, (int) n_r);
 }
 
 // Voxels from which the partitioned form is the faster one, with at most kFewParts partitions
@@ -1052,11 +1111,11 @@ extern "C" int maxi_field_histogram(const uint16_t *voxels, int64_t nZ, int64_t 
         xmap[X] = (uint32_t) std::min<int64_t>(nx - 1, (int64_t) std::floor((double) t));
     }
     xmap.resize(round_up(nX, kVec), 0);
-    DeviceTables t;
+    HostTables t;
     const size_t o_vT = t.add(vT.data(), vT.size()), o_fT = t.add(fT.data(), fT.size());
     const size_t o_z = t.add(zmap.data(), zmap.size()), o_y = t.add(ymap.data(), ymap.size());
     const size_t o_x = t.add(xmap.data(), xmap.size());
-    const size_t tables = (t.host.size() * sizeof(uint32_t) + 255) / 256 * 256;
+    const size_t tables = (t.bytes() + 255) / 256 * 256;
     FieldPlan f = field_plan(nZ, nY, nX, field_bins, voxel_bins, tables);
     SpareBuffer scratch;
     rc = scratch.take(f.bytes, st, "histogram");
@@ -1066,8 +1125,7 @@ extern "C" int maxi_field_histogram(const uint16_t *voxels, int64_t nZ, int64_t 
         rc = scratch.take(tables, st, "histogram");
     }
     if (rc) return rc;
-    cudaError_t e =
-        cudaMemcpyAsync(scratch.data(), t.host.data(), t.host.size() * sizeof(uint32_t), cudaMemcpyHostToDevice, st);
+    const cudaError_t e = t.copy_to(scratch.data(), st);
     if (e != cudaSuccess) return set_cuda_error(e, "histogram tables");
     const uint32_t *dev = reinterpret_cast<const uint32_t *>(scratch.data());
     if (!vT.empty()) vm.T = dev + o_vT;
@@ -1105,11 +1163,7 @@ extern "C" int maxi_field_histogram(const uint16_t *voxels, int64_t nZ, int64_t 
             field_histogram_kernel<false><<<grid, 256, 0, st>>>(voxels, field, nZ, nY, (int) nX, ny, nx, y_start,
                                                                 (int) x_start, vm, fm, zm, ym, xm, b, voxel_bins);
     }
-    e = rc == MAXI_OK ? cudaGetLastError() : cudaSuccess;
-    const cudaError_t e2 = scratch.give_back();  // waits for the stream: the host tables are free after it
-    if (rc) return rc;
-    if (e == cudaSuccess) e = e2;
-    return e == cudaSuccess ? MAXI_OK : set_cuda_error(e, "field histogram");
+    return finish(scratch, st, rc, "field histogram");
 }
 
 extern "C" int maxi_axis_histograms(const uint16_t *voxels, int64_t nz_block, int64_t Nz, int64_t Ny, int64_t Nx,
@@ -1138,16 +1192,19 @@ extern "C" int maxi_axis_histograms(const uint16_t *voxels, int64_t nz_block, in
     std::vector<uint32_t> vT;
     BinMap vm{};
     if ((rc = cached_bin_map(true, vmin, vmax, voxel_bins, vT, vm))) return rc;
-    DeviceTables t;
-    const size_t o_vT = t.add(vT.data(), vT.size());
-    rc = upload(t, st);
-    if (rc == MAXI_OK) {
-        if (!vT.empty()) vm.T = t.dev + o_vT;
-        auto *xb = reinterpret_cast<unsigned long long *>(x_bins), *yb = reinterpret_cast<unsigned long long *>(y_bins);
-        auto *zb = reinterpret_cast<unsigned long long *>(z_bins), *rb = reinterpret_cast<unsigned long long *>(r_bins);
-        const bool vec = Nx % kVec == 0 && reinterpret_cast<uintptr_t>(voxels) % 16 == 0;
-        rc = axis_launches(voxels, nzl, Ny, (int) Nx, z_start, y_start, (int) x_start, vm, cy, cx, xb, yb, zb, rb,
-                           (int) voxel_bins, n_r, vec, std::max(rx, ry), st);
+    HostTables t;
+    t.add(vT.data(), vT.size());
+    SpareBuffer scratch;
+    if (!vT.empty()) {
+        if ((rc = scratch.take(t.bytes(), st, "histogram"))) return rc;
+        const cudaError_t e = t.copy_to(scratch.data(), st);
+        if (e != cudaSuccess) return set_cuda_error(e, "histogram tables");
+        vm.T = reinterpret_cast<const uint32_t *>(scratch.data());
     }
-    return finish(t, st, rc, "axis histograms");
+    auto *xb = reinterpret_cast<unsigned long long *>(x_bins), *yb = reinterpret_cast<unsigned long long *>(y_bins);
+    auto *zb = reinterpret_cast<unsigned long long *>(z_bins), *rb = reinterpret_cast<unsigned long long *>(r_bins);
+    const bool vec = Nx % kVec == 0 && reinterpret_cast<uintptr_t>(voxels) % 16 == 0;
+    rc = axis_launches(voxels, nzl, Ny, (int) Nx, z_start, y_start, (int) x_start, vm, cy, cx, xb, yb, zb, rb,
+                       (int) voxel_bins, n_r, vec, std::max(rx, ry), st);
+    return finish(scratch, st, rc, "axis histograms");
 }
