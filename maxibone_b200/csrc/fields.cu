@@ -125,25 +125,26 @@ __global__ void __launch_bounds__(256) field_maxima(const uint16_t *__restrict__
     }
 }
 
-// The walk of the other two passes: `lanes` (a power of two) threads per row, 8 voxels each
-// at a time (VEC: rows are 16-byte aligned) or one; row(r) for every row, then
-// voxels(r, x, a, b) with the two fields' voxels from x on.  Row indices stay below
-// 2^32 (the host checks), so their division is 32-bit.
+// The walk of the other two passes: `lanes` (a power of two; of all the launch's threads in order)
+// threads per row, 8 voxels each at a time (VEC: rows are 16-byte aligned) or one; row(r) for
+// every row, then voxels(r, x, a, b) with the two fields' voxels from x on.  Row indices stay
+// below 2^32 (the host checks), so their division is 32-bit.  A warp to a row, or more threads where
+// there are too few rows for the chip (1 x 4 x 4194304: the two passes 11.7 ms with a warp, 0.04 now).
 template <bool VEC, typename Row, typename Voxels>
 __device__ __forceinline__ void for_rows(const uint16_t *__restrict__ g, const uint16_t *__restrict__ e, int64_t rows,
-                                         int nx, int lanes, Row &&row, Voxels &&voxels) {
+                                         uint32_t nx, int lanes, Row &&row, Voxels &&voxels) {
     constexpr int V = VEC ? 8 : 1, kAtOnce = VEC ? 2 : 4;
-    const int lane = threadIdx.x & (lanes - 1);
-    const int64_t first = ((int64_t) blockIdx.x * blockDim.x + threadIdx.x) / lanes;
+    const int thread = blockIdx.x * blockDim.x + threadIdx.x, lane = thread & (lanes - 1);
+    const int64_t first = thread / lanes;
     const int64_t step = (int64_t) gridDim.x * blockDim.x / lanes;
     for (int64_t r = first; r < rows; r += step) {
         row(r);
         const uint16_t *gr = g + r * nx, *er = e + r * nx;
-        for (int x0 = lane * V; x0 < nx; x0 += kAtOnce * lanes * V) {
+        for (uint32_t x0 = lane * V; x0 < nx; x0 += kAtOnce * lanes * V) {
             uint4 a[kAtOnce], b[kAtOnce];
 #pragma unroll
             for (int k = 0; k < kAtOnce; k++) {
-                const int x = x0 + k * lanes * V;
+                const uint32_t x = x0 + k * lanes * V;
                 if (x < nx) {
                     if (VEC) {
                         a[k] = __ldg(reinterpret_cast<const uint4 *>(gr + x));
@@ -156,25 +157,26 @@ __device__ __forceinline__ void for_rows(const uint16_t *__restrict__ g, const u
             }
 #pragma unroll
             for (int k = 0; k < kAtOnce; k++) {
-                const int x = x0 + k * lanes * V;
+                const uint32_t x = x0 + k * lanes * V;
                 if (x < nx) voxels(r, x, a[k], b[k]);
             }
+            if (nx - x0 <= (uint32_t) (kAtOnce * lanes * V)) break;  // (x0 may be about to wrap around)
         }
     }
 }
 // Extremes of c = G / gm - E / em with numpy's FP32 operations (no contraction).
 template <bool VEC>
 __global__ void __launch_bounds__(256) combined_extremes(const uint16_t *__restrict__ g, const uint16_t *__restrict__ e,
-                                                         int64_t rows, uint32_t ny, int nx, int lanes,
-                                                         const int2 *__restrict__ inside, CombineStats *st) {
+                                                         int64_t rows, uint32_t ny, uint32_t nx, int lanes,
+                                                         const uint2 *__restrict__ inside, CombineStats *st) {
     constexpr int V = VEC ? 8 : 1;
     if (st->gmax == 0 || st->emax == 0) return;  // the host reports it
     const Divisor by_g = divisor((float) st->gmax), by_e = divisor((float) st->emax);
     const float inf = __int_as_float(0x7f800000);
     float lo = inf, hi = -inf, lo_in = inf, hi_in = -inf;
-    int2 iv = make_int2(0, 0);
+    uint2 iv = make_uint2(0, 0);
     for_rows<VEC>(g, e, rows, nx, lanes, [&](int64_t r) { iv = __ldg(inside + (uint32_t) r % ny); },
-                  [&](int64_t, int x, const uint4 &wa, const uint4 &wb) {
+                  [&](int64_t, uint32_t x, const uint4 &wa, const uint4 &wb) {
                       const uint32_t a[4] = {wa.x, wa.y, wa.z, wa.w}, b[4] = {wb.x, wb.y, wb.z, wb.w};
                       float c[V + 1], l = inf, h = -inf;
 #pragma unroll
@@ -215,8 +217,9 @@ __global__ void __launch_bounds__(256) combined_extremes(const uint16_t *__restr
 // any_inside / any_outside: whether the cylinder has voxels, and whether some are outside it.
 template <bool VEC>
 __global__ void __launch_bounds__(256) combined_convert(const uint16_t *__restrict__ g, const uint16_t *__restrict__ e,
-                                                        uint16_t *__restrict__ out, int64_t rows, uint32_t ny, int nx,
-                                                        int lanes, const int2 *__restrict__ inside, bool any_inside,
+                                                        uint16_t *__restrict__ out, int64_t rows, uint32_t ny,
+                                                        uint32_t nx, int lanes, const uint2 *__restrict__ inside,
+                                                        bool any_inside,
                                                         bool any_outside, const CombineStats *__restrict__ st) {
     constexpr int V = VEC ? 8 : 1;
     if (st->gmax == 0 || st->emax == 0) return;
@@ -236,10 +239,10 @@ __global__ void __launch_bounds__(256) combined_convert(const uint16_t *__restri
     const bool some = by_range.b > 0.0f;
     auto walk = [&](auto plain) {
         constexpr bool PLAIN = decltype(plain)::value;
-        int2 iv = make_int2(0, 0);
+        uint2 iv = make_uint2(0, 0);
         for_rows<VEC>(
             g, e, rows, nx, lanes, [&](int64_t r) { iv = __ldg(inside + (uint32_t) r % ny); },
-            [&](int64_t r, int x, const uint4 &wa, const uint4 &wb) {
+            [&](int64_t r, uint32_t x, const uint4 &wa, const uint4 &wb) {
                 const uint32_t a[4] = {wa.x, wa.y, wa.z, wa.w}, b[4] = {wb.x, wb.y, wb.z, wb.w};
                 uint32_t q[4] = {0u, 0u, 0u, 0u};
                 if (some && x + V > iv.x && x < iv.y) {
@@ -282,7 +285,7 @@ double linspace_pm1(int64_t i, int64_t n) {
 // xs[x]^2 + ys[y]^2 < 1 in FP64.  xs^2 falls then rises along x and fl(a + c) is
 // monotone in a, so a row's inside voxels run from a first to a last index around
 // the argmin of xs^2: two binary searches per row, exact.
-void cylinder_intervals(int64_t ny, int64_t nx, std::vector<int2> &inside, bool &any_outside, bool &any_inside) {
+void cylinder_intervals(int64_t ny, int64_t nx, std::vector<uint2> &inside, bool &any_outside, bool &any_inside) {
     std::vector<double> xs2(nx);
     int64_t xm = 0;
     for (int64_t x = 0; x < nx; x++) {
@@ -291,7 +294,7 @@ void cylinder_intervals(int64_t ny, int64_t nx, std::vector<int2> &inside, bool 
         xs2[x] = sq;
         if (xs2[x] < xs2[xm]) xm = x;
     }
-    inside.assign(ny, make_int2(0, 0));
+    inside.assign(ny, make_uint2(0, 0));
     any_outside = any_inside = false;
     for (int64_t y = 0; y < ny; y++) {
         const double v = linspace_pm1(y, ny);
@@ -317,7 +320,7 @@ void cylinder_intervals(int64_t ny, int64_t nx, std::vector<int2> &inside, bool 
             }
             x1 = lo;
         }
-        inside[y] = make_int2((int) x0, (int) x1);
+        inside[y] = make_uint2((uint32_t) x0, (uint32_t) x1);
         any_outside |= x0 > 0 || x1 < nx;
         any_inside |= x1 > x0;
     }
@@ -326,12 +329,12 @@ void cylinder_intervals(int64_t ny, int64_t nx, std::vector<int2> &inside, bool 
 // Zeroes the voxels of each row outside its cylinder interval (one block per row
 // at a time; the inside voxels are neither read nor written).
 __global__ void cylinder_zero(uint16_t *__restrict__ f, int64_t rows, int64_t ny, int nx,
-                              const int2 *__restrict__ iv) {
+                              const uint2 *__restrict__ iv) {
     for (int64_t row = blockIdx.x; row < rows; row += gridDim.x) {
-        const int2 in = __ldg(iv + row % ny);
+        const uint2 in = __ldg(iv + row % ny);
         uint16_t *r = f + row * nx;
-        for (int x = threadIdx.x; x < in.x; x += blockDim.x) r[x] = 0;
-        for (int x = in.y + threadIdx.x; x < nx; x += blockDim.x) r[x] = 0;
+        for (int x = threadIdx.x; x < (int) in.x; x += blockDim.x) r[x] = 0;
+        for (int x = (int) in.y + threadIdx.x; x < nx; x += blockDim.x) r[x] = 0;
     }
 }
 
@@ -354,15 +357,15 @@ extern "C" int maxi_combine_fields(const uint16_t *gauss, const uint16_t *edt, i
     if (rows * nx >= (int64_t(1) << 32))
         return set_error(MAXI_ERR_UNSUPPORTED, "volumes of 2^32 voxels or more are not served by this step");
 
-    std::vector<int2> inside;
+    std::vector<uint2> inside;
     bool any_outside = false, any_inside = false;
     cylinder_intervals(ny, nx, inside, any_outside, any_inside);
 
-    const size_t iv_bytes = (size_t) ny * sizeof(int2);
+    const size_t iv_bytes = (size_t) ny * sizeof(uint2);
     SpareBuffer scratch;
     if ((rc = scratch.take(256 + iv_bytes, st, "field combination"))) return rc;
     CombineStats *d_st = reinterpret_cast<CombineStats *>(scratch.data());
-    int2 *d_iv = reinterpret_cast<int2 *>(scratch.data() + 256);
+    uint2 *d_iv = reinterpret_cast<uint2 *>(scratch.data() + 256);
     const bool aligned = ((reinterpret_cast<uintptr_t>(gauss) | reinterpret_cast<uintptr_t>(edt) |
                            reinterpret_cast<uintptr_t>(output)) & 15) == 0;
     const bool vec = nx % 8 == 0 && aligned;
@@ -371,9 +374,13 @@ extern "C" int maxi_combine_fields(const uint16_t *gauss, const uint16_t *edt, i
     cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
     const int threads = 256;
     int lanes = 1;
-    while (lanes < 32 && lanes * (vec ? 8 : 1) < nx) lanes *= 2;
+    // (At least 64 voxels a thread: every warp ends in four additions to the same words.)
+    const int64_t wanted = std::min<int64_t>((int64_t) sms * 1024, rows * nx / 64);
+    while (lanes * (vec ? 8 : 1) < nx && (lanes < 32 || rows * lanes < wanted)) lanes *= 2;
     const unsigned grid_flat = (unsigned) std::min<int64_t>(ceil_div(ceil_div(rows * nx, 8), threads), (int64_t) sms * 16);
-    const unsigned grid = (unsigned) std::min<int64_t>(ceil_div(rows * lanes, threads), (int64_t) sms * 16);
+    // (Of more lanes than a block has threads, whole rows: the grid is a multiple of lanes / threads.)
+    const int64_t blocks = std::min<int64_t>(ceil_div(rows * lanes, threads), (int64_t) sms * 16);
+    const unsigned grid = (unsigned) (lanes > threads ? round_up(blocks, lanes / threads) : blocks);
     CombineStats pageable{};
     const StagingBuffer staging;
     CombineStats &h = staging.data() ? *static_cast<CombineStats *>(staging.data()) : pageable;
@@ -382,10 +389,10 @@ extern "C" int maxi_combine_fields(const uint16_t *gauss, const uint16_t *edt, i
     if (e == cudaSuccess) {
         field_maxima<<<grid_flat, threads, 0, st>>>(gauss, edt, rows * nx, aligned, d_st);
         auto extremes = vec ? combined_extremes<true> : combined_extremes<false>;
-        extremes<<<grid, threads, 0, st>>>(gauss, edt, rows, (uint32_t) ny, (int) nx, lanes, d_iv, d_st);
+        extremes<<<grid, threads, 0, st>>>(gauss, edt, rows, (uint32_t) ny, (uint32_t) nx, lanes, d_iv, d_st);
         auto convert = vec ? combined_convert<true> : combined_convert<false>;
-        convert<<<grid, threads, 0, st>>>(gauss, edt, output, rows, (uint32_t) ny, (int) nx, lanes, d_iv, any_inside,
-                                          any_outside, d_st);
+        convert<<<grid, threads, 0, st>>>(gauss, edt, output, rows, (uint32_t) ny, (uint32_t) nx, lanes, d_iv,
+                                          any_inside, any_outside, d_st);
         e = cudaGetLastError();
     }
     if (e == cudaSuccess) e = cudaMemcpyAsync(&h, d_st, sizeof(h), cudaMemcpyDeviceToHost, st);
@@ -408,12 +415,12 @@ extern "C" int maxi_mask_cylinder(uint16_t *field, int64_t nz, int64_t ny, int64
     int rc = require_device();
     if (rc) return rc;
     cudaStream_t st = static_cast<cudaStream_t>(stream);
-    std::vector<int2> inside;
+    std::vector<uint2> inside;
     bool any_outside = false, any_inside = false;
     cylinder_intervals(ny, nx, inside, any_outside, any_inside);
     if (!any_outside) return MAXI_OK;
-    int2 *d_iv = nullptr;
-    const size_t bytes = inside.size() * sizeof(int2);
+    uint2 *d_iv = nullptr;
+    const size_t bytes = inside.size() * sizeof(uint2);
     if (cudaMallocAsync(reinterpret_cast<void **>(&d_iv), bytes, st) != cudaSuccess) {
         cudaGetLastError();
         return set_error(MAXI_ERR_OUT_OF_MEMORY, "could not allocate %zu bytes of intervals", bytes);

@@ -704,14 +704,13 @@ __device__ __forceinline__ int isqrt32(int n) {
 template <bool EXACT, bool SPLIT>
 __global__ void __launch_bounds__(1024) ring_histograms(const uint16_t *__restrict__ voxels, int64_t nzl, int Ny,
                                                         int Nx, int y_start, int x_start, BinMap vm, int cy, int cx,
-                                                        int rings, int width, int64_t per, int parts,
+                                                        int rings, int width, int64_t per, int chunks,
+                                                        int parts,
                                                         unsigned long long *__restrict__ r_bins, int voxel_bins,
                                                         int n_r) {
     extern __shared__ uint32_t counters[];
-    const int64_t chunks = (nzl + per - 1) / per;
-    const int part = (int) (blockIdx.x % parts);
-    const int ring = rings - 1 - (int) (blockIdx.x / parts / chunks);
-    const int64_t z0 = blockIdx.x / parts % chunks * per;
+    const int b = (int) blockIdx.x, part = b % parts, chunk = b / parts % chunks, ring = rings - 1 - b / parts / chunks;
+    const int64_t z0 = chunk * per;
     const int planes = (int) min(per, nzl - z0);
     const int r0 = ring * width, r1 = min(r0 + width, n_r);
     counters_clear(counters, (r1 - r0) * voxel_bins);
@@ -985,14 +984,15 @@ int axis_launches(const uint16_t *voxels, int64_t nzl, int64_t Ny, int Nx, int64
         if (rings * chunks * parts >= sms * 3 / 4 || width <= kVec) break;
     }
     const int64_t per = ceil_div(nzl, chunks);
+    chunks = ceil_div(nzl, per);
     // Rows that a ring of half the largest radius meets.
     const double half = 0.5 * (double) radii, widest = (double) std::max(std::abs(x_start - cx), std::abs(Nx - 1 - cx));
     const double low = std::sqrt(std::max(0.0, half * half - widest * widest));
     const bool split = per <= 2 || 2.0 * (half + (double) width - low) < 64.0 || Ny < 64;
     auto kernel = split ? (exact ? ring_histograms<true, true> : ring_histograms<false, true>)
                         : (exact ? ring_histograms<true, false> : ring_histograms<false, false>);
-    return launch(kernel, rings * ceil_div(nzl, per) * parts, 1024, (int) width * voxel_bins, voxels, nzl, (int) Ny, Nx,
-                  (int) y_start, x_start, vm, (int) cy, (int) cx, (int) rings, (int) width, per, (int) parts, rb,
+    return launch(kernel, rings * chunks * parts, 1024, (int) width * voxel_bins, voxels, nzl, (int) Ny, Nx,
+                  (int) y_start, x_start, vm, (int) cy, (int) cx, (int) rings, (int) width, per, (int) chunks, (int) parts, rb,
                   voxel_bins, (int) n_r);
 }
 
