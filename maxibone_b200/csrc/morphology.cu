@@ -246,14 +246,24 @@ __global__ void morph_combine(const Partials p, uint32_t *__restrict__ out, int6
     }
 }
 
-// uint8 result.  A warp combines 32 words and writes them out together: 16 bytes per lane
-// (VEC: rows are whole words and 16-byte aligned), or a word's 32 voxels at a time.
+// Words that a warp takes at a time where it handles a word's 32 voxels in one step: 32, or fewer
+// for volumes that would leave warps idle (16^3: packing 8.7 us with 32, 1.7 with 1).
+int words_per_warp(int64_t words, int64_t warps) {
+    int n = 32;
+    while (n > 1 && ceil_div(words, n) < warps) n /= 2;
+    return n;
+}
+
+// uint8 result.  A warp combines `per` words (32 or a smaller power of two) and writes them out
+// together: 16 bytes per lane (VEC: rows are whole words and 16-byte aligned, 32 words), or a word's 32
+// voxels at a time.
 template <bool DILATE, bool VEC>
-__global__ void morph_combine_u8(const Partials p, uint8_t *__restrict__ out, int64_t words, int nx, int nw) {
+__global__ void morph_combine_u8(const Partials p, uint8_t *__restrict__ out, int64_t words, int nx, int nw, int per) {
     const int lane = threadIdx.x & 31;
-    const int64_t stride = (int64_t) gridDim.x * blockDim.x;
-    for (int64_t first = ((int64_t) blockIdx.x * blockDim.x + threadIdx.x) & ~31; first < words; first += stride) {
-        const WordAt at(min(first + lane, words - 1), p.ny, nw);
+    if (VEC) per = 32;
+    const int64_t stride = (int64_t) gridDim.x * blockDim.x / 32 * per;
+    for (int64_t first = ((int64_t) blockIdx.x * blockDim.x + threadIdx.x) / 32 * per; first < words; first += stride) {
+        const WordAt at(min(first + (VEC ? lane : min(lane, per - 1)), words - 1), p.ny, nw);
         const uint32_t word = combined_word<DILATE>(p, at);
         const uint32_t bits = __brev(word);  // bit q: voxel q
         if (VEC) {
@@ -270,7 +280,7 @@ __global__ void morph_combine_u8(const Partials p, uint8_t *__restrict__ out, in
             }
         } else {
             const int x = at.x * 32;
-            for (int k = 0; k < 32 && first + k < words; k++) {
+            for (int k = 0; k < per && first + k < words; k++) {
                 const uint32_t b = __shfl_sync(0xffffffffu, bits, k);
                 const int64_t r = __shfl_sync(0xffffffffu, at.row, k);
                 const int xk = __shfl_sync(0xffffffffu, x, k) + lane;
@@ -282,10 +292,10 @@ __global__ void morph_combine_u8(const Partials p, uint8_t *__restrict__ out, in
 
 // uint8 rows -> packed words (MSB first), padding bits neutral.  VEC: rows are whole words
 // (nx % 32 == 0) and 16-byte aligned, one thread per word with two 16-byte loads; otherwise
-// a warp takes 32 words, a word's 32 voxels at a time.
+// a warp takes `per` words, a word's 32 voxels at a time.
 template <bool DILATE, bool VEC>
 __global__ void morph_pack(const uint8_t *__restrict__ in, uint32_t *__restrict__ packed, int64_t words, int nx,
-                           int nw) {
+                           int nw, int per) {
     const int64_t stride = (int64_t) gridDim.x * blockDim.x, thread = (int64_t) blockIdx.x * blockDim.x + threadIdx.x;
     if (VEC) {
         for (int64_t idx = thread; idx < words; idx += stride) {
@@ -303,10 +313,10 @@ __global__ void morph_pack(const uint8_t *__restrict__ in, uint32_t *__restrict_
         return;
     }
     const int lane = threadIdx.x & 31;
-    for (int64_t first = thread & ~31; first < words; first += stride) {
+    for (int64_t first = thread / 32 * per; first < words; first += stride / 32 * per) {
         uint32_t mine = 0;
 #pragma unroll 8
-        for (int k = 0; k < 32; k++) {
+        for (int k = 0; k < per; k++) {
             const WordAt at(min(first + k, words - 1), 1, nw);
             const int x = at.x * 32 + lane;
             bool bit = !DILATE;
@@ -317,7 +327,7 @@ __global__ void morph_pack(const uint8_t *__restrict__ in, uint32_t *__restrict_
             const uint32_t word = __brev(__ballot_sync(0xffffffffu, bit));
             if (lane == k) mine = word;
         }
-        if (first + lane < words) packed[first + lane] = mine;
+        if (lane < per && first + lane < words) packed[first + lane] = mine;
     }
 }
 
@@ -362,7 +372,8 @@ int morph_kernel(int radius, void (**kernel)(const uint32_t *, uint32_t *, const
 // ends first, counting rounds of resident blocks and about one plane's time to start and
 // finish a block.  It is small volumes that this is for (128^3, r = 8: 44 us with 2 planes
 // per block, 134 with 32, which leave 16 blocks); large ones are even from 16 planes on.  At
-// least two planes: the scratch then stays within (radius + 1) words per word.
+// least two planes: the scratch then stays within (radius + 1) words per word, of rows rounded up to
+// 4 words.
 MorphTile morph_tile(int64_t nz, int64_t ny, int64_t nw, int radius, int pmax, int resident) {
     MorphTile t{};
     t.nw = (int) nw;
@@ -383,8 +394,11 @@ MorphTile morph_tile(int64_t nz, int64_t ny, int64_t nw, int radius, int pmax, i
     fill_pairs(t, radius, tile_words(rb) * 4);
     return t;
 }
+// The scratch: `radius` planes that reach over each cut between two blocks, from either side.  The
+// first block's planes below 0 and the last one's above the volume are never written, so that the
+// layout starts with the first block's plane `radius`.
 int64_t partial_words(const MorphTile &t) {
-    return (int64_t) t.blocks * (t.planes + 2 * t.radius) * t.ny * t.pitch;
+    return (t.nz + 2 * (int64_t) t.radius * (t.blocks - 1)) * t.ny * t.pitch;
 }
 Partials partials(const MorphTile &t, const uint32_t *words) {
     return {words, t.nz, t.ny, t.pitch, t.radius, t.planes};
@@ -414,17 +428,19 @@ int morph_run(const void *in, void *out, int64_t nz, int64_t ny, int64_t nx, int
     const int64_t packed_words = U8 ? round_up(words, 4) : 0;
     uint32_t *scratch = nullptr;
     if ((rc = acquire_scratch((size_t) (packed_words + partial_words(t)) * sizeof(uint32_t), hold, &scratch, "morphology"))) return rc;
-    uint32_t *partial = scratch + packed_words;
+    uint32_t *partial = scratch + packed_words - (int64_t) t.radius * t.ny * t.pitch;
     const unsigned g = grid_for(words);
     if constexpr (U8) {
         const bool vec = nx % 32 == 0 && ((reinterpret_cast<uintptr_t>(in) | reinterpret_cast<uintptr_t>(out)) & 15) == 0;
         const uint8_t *src = static_cast<const uint8_t *>(in);
         uint8_t *dst = static_cast<uint8_t *>(out);
-        if (vec) morph_pack<DILATE, true><<<g, 256, 0, st>>>(src, scratch, words, (int) nx, t.nw);
-        else morph_pack<DILATE, false><<<g, 256, 0, st>>>(src, scratch, words, (int) nx, t.nw);
+        const int per = words_per_warp(words, 148 * 16);
+        const unsigned gw = grid_for(ceil_div(words, per) * 32);
+        if (vec) morph_pack<DILATE, true><<<g, 256, 0, st>>>(src, scratch, words, (int) nx, t.nw, 1);
+        else morph_pack<DILATE, false><<<gw, 256, 0, st>>>(src, scratch, words, (int) nx, t.nw, per);
         if ((rc = morph_partial_planes<DILATE>(scratch, partial, t, kernel, st))) return rc;
-        if (vec) morph_combine_u8<DILATE, true><<<g, 256, 0, st>>>(partials(t, partial), dst, words, (int) nx, t.nw);
-        else morph_combine_u8<DILATE, false><<<g, 256, 0, st>>>(partials(t, partial), dst, words, (int) nx, t.nw);
+        if (vec) morph_combine_u8<DILATE, true><<<g, 256, 0, st>>>(partials(t, partial), dst, words, (int) nx, t.nw, 32);
+        else morph_combine_u8<DILATE, false><<<gw, 256, 0, st>>>(partials(t, partial), dst, words, (int) nx, t.nw, per);
     } else {
         if ((rc = morph_partial_planes<DILATE>(static_cast<const uint32_t *>(in), partial, t, kernel, st))) return rc;
         morph_combine<DILATE><<<g, 256, 0, st>>>(partials(t, partial), static_cast<uint32_t *>(out), words, t.nw);
