@@ -44,35 +44,38 @@ cudaError_t axis_pass(const float *in, const uint32_t *mask, float *out, int64_t
     return launch_pass(kernel, true, outer * s.col_tiles * s.segments, kStreamThreads, s.ring * kStreamRow, st, in, mask, out, s, taps);
 }
 
-// The tile form of the x pass (contig_pass): 16-byte copies and unrolled taps.
-template <int R, int MASK_FMT, bool FINAL>
-cudaError_t x_tile_pass(const float *in, float *out, const void *mask, uint16_t *out_u16, float *field_out,
-                        int64_t rows, int64_t nx, const float *kernel, cudaStream_t st) {
+// The tile form of the x pass (contig_pass): 16-byte copies and taps unrolled for radius R, zero
+// beyond the kernel's own.
+template <int R>
+cudaError_t x_tile_pass(const float *in, float *out, const void *mask, int64_t rows, int64_t nx, int radius,
+                        const float *kernel, cudaStream_t st) {
     const int64_t xt = ceil_div(nx, kConTX);
-    return launch_pass(contig_pass<R, float, MASK_FMT, FINAL>, true, xt * ceil_div(rows, kConTR), kConThreads,
-                       contig_smem_bytes<R>(), st, in, out, mask, out_u16, field_out, rows, nx, xt,
-                       make_taps<R>(kernel, R));
+    return launch_pass(contig_pass<R, float, MAXI_MASK_BITPACKED, false>, true, xt * ceil_div(rows, kConTR), kConThreads,
+                       contig_smem_bytes<R>(), st, in, out, mask, static_cast<uint16_t *>(nullptr),
+                       static_cast<float *>(nullptr), rows, nx, xt, make_taps<R>(kernel, radius));
 }
 
-// The tile form needs rows and outputs that allow 16-byte accesses, and a radius that it is
-// unrolled for.  There it is the faster one on large volumes (1024^3: 1.50 / 1.85 / 2.76 ms
-// at r = 4 / 12 / 32 against 1.78 / 1.98 / 2.92 ms of stream_x_pass: its 16-byte copies and
-// 40 warps per SM against 4-byte copies and 20); from 256^3 down the two are even (55 us at
-// r = 32) and below that the streaming form's smaller blocks win (128^3: 7.7 against 8.8 us).
+// The tile form needs rows that allow 16-byte accesses; a uint8 mask, which only the
+// allocation-free call passes in, never comes with a volume large enough for it.  At large
+// volumes it is the faster one for all but the last repetition where at most three taps a side
+// are padding (its 16-byte copies and 40 warps per SM against 4-byte copies and 20).  1024^3, ms
+// a pass, tile against stream_x_pass: r = 5 to 8 1.69 against 1.77 to 1.80, 9 to 12 1.94 to 2.00 against
+// 2.06 to 2.12, 16 2.10 against 2.29 and more, 23 2.51 against 2.58, 29 2.84 against 2.89, 32 2.79
+// against 3.05; r = 20 2.55 against 2.43, 28 2.84 against 2.83.  The last repetition's streaming form
+// wins at every radius (r = 8 1.75 against 1.87, 32 3.05 against 3.24).  From 256^3 down the two are even
+// (58 us at r = 32) and below that the streaming form's smaller blocks win (128^3: 7.7 against 8.8).
 constexpr int64_t kTileMinVoxels = int64_t(1) << 24;
+constexpr int kTilePadding = 3;
 
 template <int MASK_FMT, bool FINAL>
 cudaError_t x_pass(const float *in, float *out, const void *mask, uint16_t *out_u16, float *field_out, int64_t rows,
                    int64_t nx, int radius, const StreamTaps &taps, cudaStream_t st) {
-    if (nx % 4 == 0 && rows * nx >= kTileMinVoxels && aligned(in, 16) &&
-        (FINAL ? aligned(out_u16, 8) && aligned(field_out, 16) : aligned(out, 16)) &&
-        (MASK_FMT == MAXI_MASK_BITPACKED || aligned(mask, 4)))
-        switch (radius) {
+    if constexpr (MASK_FMT == MAXI_MASK_BITPACKED && !FINAL)
+        if (radius > 0 && nx % 4 == 0 && rows * nx >= kTileMinVoxels && aligned(in, 16) && aligned(out, 16)) {
 #define MAXI_CASE(R) \
-    case R: return x_tile_pass<R, MASK_FMT, FINAL>(in, out, mask, out_u16, field_out, rows, nx, taps.k, st);
+    if (radius <= R && radius + kTilePadding >= R) return x_tile_pass<R>(in, out, mask, rows, nx, radius, taps.k, st);
             MAXI_CASE(4) MAXI_CASE(8) MAXI_CASE(12) MAXI_CASE(16) MAXI_CASE(24) MAXI_CASE(32)
 #undef MAXI_CASE
-        default: break;
         }
     const StreamShape s = stream_shape(1, nx, rows, kStreamRowsX, kStreamChunkX, 32, radius);
     const int smem = kStreamRowsX * stream_x_pitch(s.ring) * 4 + kStreamMaskBytes;
@@ -95,8 +98,8 @@ cudaError_t dispatch_unrolled<float>(const Volume &v, const void *mask, int mask
     cudaError_t e;
     // The first z pass reads a bit-packed mask itself; a field to continue from or a uint8
     // mask becomes the field first.
-    const bool from_mask = !o.init_field && mask_fmt == MAXI_MASK_BITPACKED;
-    if (!from_mask) {
+    const bool from_mask = !o.field_ready && !o.init_field && mask_fmt == MAXI_MASK_BITPACKED;
+    if (!from_mask && !o.field_ready) {
         ProfScope ps(MAXI_KERNEL_INIT, st);
         if (o.init_field)
             field_from_f32<float><<<std::min<int64_t>(ceil_div(v.n(), 256), 148 * 64), 256, 0, st>>>(o.init_field, buf0, v.n());
