@@ -36,6 +36,7 @@
 // each, x 155 (half of each 32-byte sector is another strip's), r 251 (a ring's row interval
 // fills about 40% of its sectors); before, one kernel with two reductions per voxel and a
 // shared histogram per row, 1611 us.
+#include <atomic>
 #include <cmath>
 #include <mutex>
 #include <type_traits>
@@ -577,10 +578,26 @@ __device__ __forceinline__ void counters_clear(uint32_t *c, int n) {
     for (int i = threadIdx.x; i < n; i += blockDim.x) c[i] = 0;
     __syncthreads();
 }
-__device__ __forceinline__ void counters_flush(const uint32_t *c, int n, unsigned long long *bins) {
+// Whether a block of voxels holds any that is counted: the z histogram, which comes first and counts
+// every voxel that the others do, then writes `call` to the word (NULL: not kept), and otherwise the
+// other kernels have nothing to do.  The word needs no clearing, as `call` differs from call to call
+// (an old value that happened to equal it would cost those kernels' time).  A block of air,
+// 128 x 1024 x 1024 at 4096 bins: 515 us with four kernels that read it, 109 now.
+struct Counted {
+    uint32_t *word;
+    uint32_t call;
+    __device__ __forceinline__ bool none() const { return word && *word != call; }
+};
+__device__ __forceinline__ void counters_flush(const uint32_t *c, int n, unsigned long long *bins,
+                                               Counted counted = Counted{}) {
     __syncthreads();
+    bool any = false;
     for (int i = threadIdx.x; i < n; i += blockDim.x)
-        if (const uint32_t k = c[i]) atomicAdd(bins + i, (unsigned long long) k);
+        if (const uint32_t k = c[i]) {
+            atomicAdd(bins + i, (unsigned long long) k);
+            any = true;
+        }
+    if (counted.word && any) *counted.word = counted.call;
 }
 
 // y_bins or z_bins: block (p, chunk) counts the rows row0(p), row0(p) + row_step, .. of one y
@@ -590,11 +607,13 @@ struct RowSets {
     int64_t sets, set_step, row_step, rows, first_row, per;  // per: rows of a chunk
     int64_t first_set;                                      // sets below are not counted
     unsigned long long *bins;                               // of set 0
+    Counted mark, counted;                                  // z: written; y: read
 };
 template <bool VEC8, bool EXACT, bool SPLIT>
 __global__ void __launch_bounds__(256) row_set_histograms(const uint16_t *__restrict__ voxels, int Nx, int x_start,
                                                           BinMap vm, RowSets s, int voxel_bins) {
     extern __shared__ uint32_t counters[];
+    if (s.counted.none()) return;
     const int64_t set = s.first_set + blockIdx.x % (s.sets - s.first_set), chunk = blockIdx.x / (s.sets - s.first_set);
     const int64_t end = min(s.rows, s.first_row + (chunk + 1) * s.per);
     const int lane = threadIdx.x & 31;
@@ -635,7 +654,7 @@ __global__ void __launch_bounds__(256) row_set_histograms(const uint16_t *__rest
             }
         }
     }
-    counters_flush(counters, voxel_bins, s.bins + set * voxel_bins);
+    counters_flush(counters, voxel_bins, s.bins + set * voxel_bins, s.mark);
 }
 
 // x_bins: block (strip, chunk) counts `strip` neighbouring x over the rows of the chunk, a
@@ -644,8 +663,9 @@ template <bool VEC8, bool EXACT>
 __global__ void __launch_bounds__(1024) strip_histograms(const uint16_t *__restrict__ voxels, int64_t rows, int64_t Ny,
                                                          int Nx, int64_t y_start, int x_start, BinMap vm, int strips,
                                                          int strip, int64_t per, unsigned long long *__restrict__ x_bins,
-                                                         int voxel_bins) {
+                                                         int voxel_bins, Counted counted) {
     extern __shared__ uint32_t counters[];
+    if (counted.none()) return;
     const int x0 = blockIdx.x % strips * strip, width = min(strip, Nx - x0), skip = max(0, x_start - x0);
     const int64_t begin = blockIdx.x / strips * per, end = min(rows, begin + per);
     counters_clear(counters, width * voxel_bins);
@@ -707,8 +727,9 @@ __global__ void __launch_bounds__(1024) ring_histograms(const uint16_t *__restri
                                                         int rings, int width, int64_t per, int chunks,
                                                         int parts,
                                                         unsigned long long *__restrict__ r_bins, int voxel_bins,
-                                                        int n_r) {
+                                                        int n_r, Counted counted) {
     extern __shared__ uint32_t counters[];
+    if (counted.none()) return;
     const int b = (int) blockIdx.x, part = b % parts, chunk = b / parts % chunks, ring = rings - 1 - b / parts / chunks;
     const int64_t z0 = chunk * per;
     const int planes = (int) min(per, nzl - z0);
@@ -920,7 +941,7 @@ constexpr int64_t kAxisMinVoxels = int64_t(1) << 17;
 int axis_launches(const uint16_t *voxels, int64_t nzl, int64_t Ny, int Nx, int64_t z_start, int64_t y_start, int x_start,
                   const BinMap &vm, int64_t cy, int64_t cx, unsigned long long *xb, unsigned long long *yb,
                   unsigned long long *zb, unsigned long long *rb, int voxel_bins, int64_t n_r, bool vec,
-                  int64_t farthest, cudaStream_t st) {
+                  int64_t farthest, Counted counted, cudaStream_t st) {
     const int64_t sms = sm_count(), rows = nzl * Ny;
     auto direct = [&](auto kernel) {
         const unsigned grid = (unsigned) std::min<int64_t>(rows, sms * 16);
@@ -940,30 +961,34 @@ int axis_launches(const uint16_t *voxels, int64_t nzl, int64_t Ny, int Nx, int64
     };
     // z and y: several chunks per plane (or y) where there are few of them, of 16 rows at least.
     auto row_sets = [&](int64_t sets, int64_t first_set, int64_t set_step, int64_t row_step, int64_t row_count,
-                        int64_t first_row, unsigned long long *bins) {
-        const int64_t n = row_count - first_row, counted = sets - first_set;
-        const int64_t chunks = std::max<int64_t>(1, std::min(ceil_div(sms * 8, counted), n / 16));
+                        int64_t first_row, unsigned long long *bins, Counted mark, Counted read) {
+        const int64_t n = row_count - first_row, n_sets = sets - first_set;
+        const int64_t chunks = std::max<int64_t>(1, std::min(ceil_div(sms * 8, n_sets), n / 16));
         const int64_t per = ceil_div(n, chunks);
-        const RowSets s{sets, set_step, row_step, row_count, first_row, per, first_set, bins};
+        const RowSets s{sets, set_step, row_step, row_count, first_row, per, first_set, bins, mark, read};
         auto kernel = [&](auto split) {
             constexpr bool S = decltype(split)::value;
             return vec ? (exact ? row_set_histograms<true, true, S> : row_set_histograms<true, false, S>)
                        : (exact ? row_set_histograms<false, true, S> : row_set_histograms<false, false, S>);
         };
-        return launch(per < 8 ? kernel(std::true_type{}) : kernel(std::false_type{}), counted * ceil_div(n, per), 256,
+        return launch(per < 8 ? kernel(std::true_type{}) : kernel(std::false_type{}), n_sets * ceil_div(n, per), 256,
                       voxel_bins, voxels, Nx, x_start, vm, s, voxel_bins);
     };
-    int rc = row_sets(nzl, 0, Ny, 1, Ny, y_start, zb + z_start * voxel_bins);
-    if (rc == MAXI_OK) rc = row_sets(Ny, y_start, 1, Ny, nzl, 0, yb);
+    int rc = row_sets(nzl, 0, Ny, 1, Ny, y_start, zb + z_start * voxel_bins, counted, Counted{});
+    if (rc == MAXI_OK) rc = row_sets(Ny, y_start, 1, Ny, nzl, 0, yb, Counted{}, counted);
     if (rc) return rc;
-    // x: strips of 8, or as many as the counters allow; chunks of at least 2048 rows.
+    // x: strips of 8, or as many as the counters allow; chunks of at least 2048 rows, and beyond a
+    // block per SM of two rows per bin, for which a block clears and flushes `strip` counters (64 x 512 x
+    // 512, 4096 bins: 167 -> 148 us a call).
     const int strip = std::min(kVec, kBlockCells / voxel_bins), strips = (int) ceil_div(Nx, strip);
-    const int64_t x_chunks = std::max<int64_t>(1, std::min(ceil_div(sms * 4, strips), rows / 2048));
+    const int64_t x_chunks = std::max<int64_t>(
+        1, std::min({ceil_div(sms * 4, strips), rows / 2048, std::max(rows / (2 * voxel_bins), sms / strips)}));
     const int64_t x_per = ceil_div(rows, x_chunks);
     const bool wide = vec && strip == kVec;
     rc = launch(wide ? (exact ? strip_histograms<true, true> : strip_histograms<true, false>)
                      : (exact ? strip_histograms<false, true> : strip_histograms<false, false>), strips * ceil_div(rows, x_per),
-                1024, strip * voxel_bins, voxels, rows, Ny, Nx, y_start, x_start, vm, strips, strip, x_per, xb, voxel_bins);
+                1024, strip * voxel_bins, voxels, rows, Ny, Nx, y_start, x_start, vm, strips, strip, x_per, xb, voxel_bins,
+                counted);
     if (rc) return rc;
     // r: rings of as many radii as the counters allow, up to 64 (a wider row interval reads no
     // fewer sectors), in chunks of 16 planes or more.  Few rings, of a volume with few bins or
@@ -974,6 +999,10 @@ int axis_launches(const uint16_t *voxels, int64_t nzl, int64_t Ny, int Nx, int64
     if (radii > 46340 - 64)  // squared distances of 2^31 in the last ring
         return direct(vec ? axis_histograms_direct<true, true> : axis_histograms_direct<false, true>);
     int64_t width = std::min<int64_t>({radii, 64, std::max(1, kBlockCells / voxel_bins)});
+    // Volumes of some extent both ways take two blocks per SM, as the rows of narrow rings are of
+    // more even length: 64 x 301 x 333, 512 bins 111 -> 102 us a call, 32 x 1024 x 1024, 512 bins 344 -> 224; of less,
+    // 1024 x 64 x 64, 64 bins 84 -> 89.
+    const int64_t enough = std::min<int64_t>(Ny, Nx) >= 128 ? sms * 2 : sms * 3 / 4, least = kVec / 2;
     int64_t rings, chunks, parts;
     for (;; width /= 2) {
         rings = ceil_div(radii, width);
@@ -981,7 +1010,7 @@ int axis_launches(const uint16_t *voxels, int64_t nzl, int64_t Ny, int Nx, int64
         const int64_t pixels = rows * Nx / (rings * chunks);
         parts = std::max<int64_t>(1, std::min({ceil_div(sms * 6, rings * chunks), ceil_div(std::min(Ny, 2 * radii), 128),
                                                pixels / (8 * width * voxel_bins)}));
-        if (rings * chunks * parts >= sms * 3 / 4 || width <= kVec) break;
+        if (rings * chunks * parts >= enough || width <= least) break;
     }
     const int64_t per = ceil_div(nzl, chunks);
     chunks = ceil_div(nzl, per);
@@ -993,7 +1022,7 @@ int axis_launches(const uint16_t *voxels, int64_t nzl, int64_t Ny, int Nx, int64
                         : (exact ? ring_histograms<true, false> : ring_histograms<false, false>);
     return launch(kernel, rings * chunks * parts, 1024, (int) width * voxel_bins, voxels, nzl, (int) Ny, Nx,
                   (int) y_start, x_start, vm, (int) cy, (int) cx, (int) rings, (int) width, per, (int) chunks, (int) parts, rb,
-                  voxel_bins, (int) n_r);
+                  voxel_bins, (int) n_r, counted);
 }
 
 // Voxels from which the partitioned form is the faster one, with at most kFewParts partitions
@@ -1195,16 +1224,24 @@ extern "C" int maxi_axis_histograms(const uint16_t *voxels, int64_t nz_block, in
     HostTables t;
     t.add(vT.data(), vT.size());
     SpareBuffer scratch;
+    static std::atomic<uint32_t> calls{0};
+    constexpr size_t kCounted = 256;  // for Counted::word
+    rc = scratch.take(kCounted + t.bytes(), st, "histogram");
+    if (rc == MAXI_ERR_OUT_OF_MEMORY && vT.empty()) {
+        clear_error();
+        rc = MAXI_OK;
+    }
+    if (rc) return rc;
     if (!vT.empty()) {
-        if ((rc = scratch.take(t.bytes(), st, "histogram"))) return rc;
-        const cudaError_t e = t.copy_to(scratch.data(), st);
+        const cudaError_t e = t.copy_to(scratch.data() + kCounted, st);
         if (e != cudaSuccess) return set_cuda_error(e, "histogram tables");
-        vm.T = reinterpret_cast<const uint32_t *>(scratch.data());
+        vm.T = reinterpret_cast<const uint32_t *>(scratch.data() + kCounted);
     }
     auto *xb = reinterpret_cast<unsigned long long *>(x_bins), *yb = reinterpret_cast<unsigned long long *>(y_bins);
     auto *zb = reinterpret_cast<unsigned long long *>(z_bins), *rb = reinterpret_cast<unsigned long long *>(r_bins);
     const bool vec = Nx % kVec == 0 && reinterpret_cast<uintptr_t>(voxels) % 16 == 0;
     rc = axis_launches(voxels, nzl, Ny, (int) Nx, z_start, y_start, (int) x_start, vm, cy, cx, xb, yb, zb, rb,
-                       (int) voxel_bins, n_r, vec, std::max(rx, ry), st);
+                       (int) voxel_bins, n_r, vec, std::max(rx, ry),
+                       Counted{reinterpret_cast<uint32_t *>(scratch.data()), ++calls}, st);
     return finish(scratch, st, rc, "axis histograms");
 }

@@ -54,3 +54,25 @@ def _time(shape, voxel_bins):
 @pytest.mark.parametrize("shape", [(1, 4096, 4096), (64, 1024, 1024)])
 def test_few_bins_take_no_longer(shape):
     assert _time(shape, 64) <= 2.0 * _time(shape, 512)
+
+
+# A block without a counted voxel ends after the first of the four histograms; one counted voxel, at
+# the block's first and last place and beside an offset, brings the others.
+@pytest.mark.parametrize("where", [None, (0, 0, 0), (11, 150, 299), (5, 3, 40)])
+@pytest.mark.parametrize("voxel_bins", [16, 4096])
+def test_blocks_with_hardly_a_counted_voxel(where, voxel_bins):
+    shape, offset = (12, 151, 300), (0, 0, 0)
+    voxels = np.zeros(shape, np.uint16)
+    voxels[::3] = 65535
+    if where == (5, 3, 40):
+        offset = (0, 3, 40)
+        voxels[:, :3] = voxels[:, :, :40] = 900
+    if where:
+        voxels[where] = 20000
+    n_r = 169
+    want = oracle.axis_histograms(voxels, offset, shape, voxel_bins, n_r, (75, 150), (1.0, 32000.0))
+    assert (want[2].sum() > 0) == bool(where)
+    got = [np.full((n, voxel_bins), 3, np.uint64) for n in (shape[2], shape[1], shape[0], n_r)]
+    axis_histograms(voxels, offset, *got, (75, 150), (1.0, 32000.0), 0)
+    for g, w, name in zip(got, want, ("x", "y", "z", "r")):
+        np.testing.assert_array_equal(g, w + np.uint64(3), err_msg=name)
