@@ -50,6 +50,15 @@ std::map<int, Spares> g_spares;
 int SpareBuffer::take(size_t bytes, cudaStream_t st, const char *what) {
     cudaError_t e = cudaGetDevice(&device_);
     if (e != cudaSuccess) return set_cuda_error(e, "cudaGetDevice");
+    // These calls wait for their stream and cannot be captured.  Refused here, as memory allocated
+    // in a capture belongs to its graph and must not come into the list.
+    cudaStreamCaptureStatus capture = cudaStreamCaptureStatusNone;
+    e = cudaStreamIsCapturing(st, &capture);
+    if (e == cudaSuccess && capture != cudaStreamCaptureStatusNone) e = cudaErrorStreamCaptureUnsupported;
+    if (e != cudaSuccess) {
+        cudaGetLastError();
+        return set_cuda_error(e, what);
+    }
     bytes = std::max(bytes, kSmallSpare);
     Spare too_small{};
     {

@@ -10,7 +10,7 @@ import torch
 
 from maxibone_b200 import _lib, diffusion, gauss_kernel
 from maxibone_b200.fields import combine_fields
-from maxibone_b200.histograms import field_histogram
+from maxibone_b200.histograms import axis_histograms, field_histogram
 
 pytestmark = pytest.mark.gpu
 
@@ -126,3 +126,44 @@ def test_in_memory_diffusion_takes_the_kept_memory_back(capfd):
     want = np.empty(shape, np.uint16)
     diffusion(mask, kernel, want, 1)
     np.testing.assert_array_equal(out, want)
+
+
+# These calls wait for their stream, so one on a stream that is being captured is refused.  It leaves no
+# memory of the capture's behind for the next call to use.
+@pytest.mark.parametrize("make", [_combination, lambda: _histogram(8), lambda: _axis()],
+                         ids=["combine", "histogram", "axis"])
+def test_refused_under_capture(make):
+    call = make()
+    want = [t.clone() for t in _tensors(call())]
+    _release()  # the refused call finds no kept buffer
+    stream = torch.cuda.Stream()
+    graph = torch.cuda.CUDAGraph()
+    torch.cuda.synchronize()
+    with torch.cuda.stream(stream):
+        graph.capture_begin()
+        try:
+            with pytest.raises(_lib.MaxiError):
+                call()
+        finally:
+            graph.capture_end()
+    del graph
+    torch.cuda.synchronize()
+    for _ in range(2):
+        for got, expected in zip(_tensors(call()), want):
+            assert torch.equal(got, expected)
+
+
+def _tensors(result):
+    return result if isinstance(result, list) else [result]
+
+
+def _axis():
+    voxels = _u16((16, 128, 128), 5, 32000)
+    bins = [torch.zeros((n, 512), dtype=torch.int64, device="cuda") for n in (128, 128, 16, 92)]
+
+    def call():
+        for b in bins:
+            b.zero_()
+        axis_histograms(voxels, (0, 0, 0), *bins, (64, 64), (1.0, 32000.0))
+        return bins
+    return call
