@@ -339,7 +339,7 @@ def fields_section(torch, np, gauss_u16, stream):
     res = {"workload": f"{shape[0]}x{shape[1]}x{shape[2]} uint16 Gaussian field (the diffusion output) + synthetic "
                        "uint16 EDT-like field", "value": vox / (ms / 1e3) / 1e9, "unit": "Gvox/s", "ms": ms,
            "hbm_gbs": alg / (ms / 1e3) / 1e9, "hbm_frac": alg / (ms / 1e3) / 1e9 / peak,
-           "alg_bytes_per_voxel": 14, "timing": "CUDA events around 5 synchronous calls (two host read-backs each)"}
+           "alg_bytes_per_voxel": 14, "timing": "CUDA events around 5 synchronous calls (one host read-back each)"}
     # The reference's own form of the step on a bounded sample: its numpy operations with
     # the reference's compiled normalized_convert (oracle/_ref), else the oracle's numpy port.
     n = 256

@@ -149,8 +149,9 @@ __global__ void field_histogram_kernel(const uint16_t *__restrict__ voxels, cons
 // its partition) by partition with counters in shared memory, lines them up there and writes
 // them out in one run; count_partitions reads them back, partition after partition.  That moves
 // the voxels once and 2 bytes a voxel each way (158 partitions of a tile: about 70 keys in a
-// row).  Bound by instruction issue (57%, 54 instructions a voxel) and the tile's barriers;
-// a branch around tiles of air made the others slower (1.90 -> 1.97 ms: it ends the overlap of
+// row).  54 instructions a voxel fill 59% of the issue slots: at 64 registers a scheduler has 7.5 warps,
+// which wait for the field's values, at the tile's barriers and in fixed latencies alike.  A
+// branch around tiles of air made the others slower (1.90 -> 1.97 ms: it ends the overlap of
 // one vector's loads with another's counting).
 // 512 x 1024 x 1024 against half resolution, 2048 x 4096 bins: 2.85 -> 1.90 ms (partition_keys
 // 1.36, count_partitions 0.50).

@@ -33,7 +33,7 @@
 //
 // Row order of the 16-bit field between repetitions.  The z pass is the only
 // pass whose tile rows lie on different planes: read from the [z][y][x] volume
-// every row of its 64 x KP box comes from another plane, and TMA delivers such
+// every row of its 64 x 128 boxes comes from another plane, and TMA delivers such
 // boxes at well under the rate of the y pass's boxes (rows one x-row apart).
 // So the x pass (which writes whole rows and can put them anywhere) stores
 // the field of every repetition but the last with its rows in [y][z][x] order,
@@ -51,7 +51,7 @@
 // accumulator, so the epilogue reads one value per voxel.
 //
 // Warp roles in a persistent CTA (one per SM): warp 0 issues TMA loads into a
-// tile ring (and L2 prefetches a few tiles ahead), warp 1 issues the MMAs (one
+// ring (the x pass also prefetches a few tiles ahead into L2), warp 1 issues the MMAs (one
 // thread) into a double-buffered TMEM accumulator, the other warps (8 in the
 // z / y passes, 16 in the x pass) drain TMEM (tcgen05.ld), narrow to the
 // storage type and store.  With error feedback on,

@@ -12,9 +12,10 @@ namespace tc {
 // halves, and a 2-stage tile ring must fit shared memory).
 constexpr int kTcMaxRadius = 32;
 // Largest radius of the single-volume tensor-core passes: the z / y passes
-// hold the Toeplitz halves in tensor memory (192 columns each at radius 128,
-// next to 64-column accumulators) and load K = 128 + 2r rows as two TMA
-// boxes; the x pass above radius 32 runs in its transposed form.
+// hold the Toeplitz set (or both halves) in tensor memory, 192 columns each at
+// radius 128, next to two 128-column accumulators (64-column ones beside both
+// halves above radius 64), and read K = 128 + 2r rows as two or three blocks of
+// 128; the x pass above radius 32 runs in its transposed form.
 constexpr int kTcMaxRadiusWide = 128;
 
 // Smallest radius served by one 16-bit coefficient set (tc_round_taps_scaled):
