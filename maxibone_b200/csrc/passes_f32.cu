@@ -66,8 +66,20 @@ cudaError_t x_tile_pass(const float *in, float *out, const void *mask, int64_t r
 // against 3.05; r = 20 2.55 against 2.43, 28 2.84 against 2.83.  The last repetition's streaming form
 // wins at every radius (r = 8 1.75 against 1.87, 32 3.05 against 3.24).  From 256^3 down the two are even
 // (58 us at r = 32) and below that the streaming form's smaller blocks win (128^3: 7.7 against 8.8).
+//
+// That is for rows that fill the tiles.  A row ends in a tile of 256 voxels or a chunk of 128, and the form
+// that computes fewer voxels beyond it gains that share: tile / stream at 2^26 voxels, r = 8, 16 and 31, at
+// nx = 64 1.54 1.81 2.09, 300 1.07 1.16 1.27, 640 1.02 1.08 1.08, 896 0.97 1.04 1.01, 1100 0.95 1.00 0.98, 700
+// 0.92 0.97 0.93, 1024 0.91 0.97 0.92.  Hence a limit on the tiles' voxels in per cent of the chunks', from whole
+// calls of 2^24 to 2^27 voxels, and with padding taps beyond radius 8 a least row: r = 14 at nx = 132
+// 1.02 times the streaming form's time, 0.98 at 200; r = 22 1.01 at 400, 0.99 at 500.
 constexpr int64_t kTileMinVoxels = int64_t(1) << 24;
 constexpr int kTilePadding = 3;
+bool rows_fill_tiles(int64_t nx, int radius, bool padded) {
+    if (padded && nx < (radius <= 8 ? 0 : radius <= 16 ? 192 : 448)) return false;
+    const int limit = radius <= 8 || (radius <= 16 && !padded) ? 115 : padded ? 106 : 112;
+    return 100 * round_up(nx, kConTX) <= limit * round_up(nx, kStreamChunkX);
+}
 
 template <int MASK_FMT, bool FINAL>
 cudaError_t x_pass(const float *in, float *out, const void *mask, uint16_t *out_u16, float *field_out, int64_t rows,
@@ -75,7 +87,8 @@ cudaError_t x_pass(const float *in, float *out, const void *mask, uint16_t *out_
     if constexpr (MASK_FMT == MAXI_MASK_BITPACKED && !FINAL)
         if (radius > 0 && nx % 4 == 0 && rows * nx >= kTileMinVoxels && aligned(in, 16) && aligned(out, 16)) {
 #define MAXI_CASE(R) \
-    if (radius <= R && radius + kTilePadding >= R) return x_tile_pass<R>(in, out, mask, rows, nx, radius, taps.k, st);
+    if (radius <= R && radius + kTilePadding >= R && rows_fill_tiles(nx, radius, radius < R)) \
+        return x_tile_pass<R>(in, out, mask, rows, nx, radius, taps.k, st);
             MAXI_CASE(4) MAXI_CASE(8) MAXI_CASE(12) MAXI_CASE(16) MAXI_CASE(24) MAXI_CASE(32)
 #undef MAXI_CASE
         }
